@@ -302,9 +302,16 @@ int svs_tvl1_plan_pair_tile_used(const svs_plan* plan, int level, int pair);
  * 2-byte fields: 40x8 voxel pairs when every width is a multiple of 40, 32x8 single voxels up to
  * width 32, 16x16 single voxels otherwise). */
 int svs_tvl1_auto_tiles(int storage, int num_pairs, const int* dims_host, int sms, int* pair_tile_out);
-/* CTAs of one iteration at a pyramid level, all variant groups together (after the first solve;
- * 0 before): the column tiles times their z chunks. */
+/* CTAs of one iteration at a pyramid level in the per-iteration form, all variant groups together
+ * (after the first solve; 0 before): the column tiles times their z chunks. */
 int64_t svs_tvl1_plan_level_ctas(const svs_plan* plan, int level);
+/* Pairs of a level whose state stays on chip (after the first solve; 0 before): each warp's
+ * iterations of these pairs run in launches of one CTA per SM that hold the pairs' volumes in
+ * registers and shared memory, faces exchanged between CTAs (bounded waits, SVS_DEV_TIMEOUT on
+ * expiry). Taken automatically where it is modelled faster than per-iteration launches (MIRROR
+ * boundary, unit spacing, no variant, chunk, persistent or stall request at the level); results
+ * are bitwise those of the split-role variants. */
+int svs_tvl1_plan_level_resident(const svs_plan* plan, int level);
 /* The z-chunk plan of the split-role kernels (host arithmetic only, no device needed): for
  * `columns` column tiles of up to `nz` planes on `slots` resident CTAs (SMs x CTAs per SM), the
  * first columns - tail_columns march in main_chunks chunks each and the last tail_columns in

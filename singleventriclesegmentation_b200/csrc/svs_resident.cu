@@ -1,0 +1,61 @@
+// Instantiations and launch of resident_kernel (svs_resident.cuh) for every storage mode and shape.
+#include "svs_resident.cuh"
+
+namespace svs {
+namespace {
+
+template <typename SU, typename SP, typename C>
+bool run(int op, unsigned grid, unsigned threads, const ResLaunch* L, const Desc* descs, const ResidentArgs* a,
+         int* status, cudaStream_t s, int* occ) {
+  const auto k = resident_kernel<SU, SP, C>;
+  if (op == 0) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, C::NT, C::SMEM) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return *occ > 0;
+  }
+  // its CTAs wait for one another: a cooperative launch starts only a grid that fits the GPU at once
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, *L, descs, *a, status) == cudaSuccess;
+}
+
+template <typename SU, typename SP>
+bool dispatch(int shape, int op, unsigned grid, unsigned threads, const ResLaunch* L, const Desc* descs,
+              const ResidentArgs* a, int* status, cudaStream_t s, int* occ) {
+  switch (shape) {
+    case 0: return run<SU, SP, ResSmall>(op, grid, threads, L, descs, a, status, s, occ);
+    case 1: return run<SU, SP, ResMid>(op, grid, threads, L, descs, a, status, s, occ);
+    case 2:
+      if constexpr (sizeof(SP) == 2) return run<SU, SP, ResLarge>(op, grid, threads, L, descs, a, status, s, occ);
+      return false;
+    default: return false;
+  }
+}
+
+}  // namespace
+
+bool resident_variant(int storage, int shape, int op, unsigned grid, unsigned threads, const ResLaunch* L,
+                      const Desc* descs, const ResidentArgs* a, int* status, cudaStream_t s, int* occ) {
+  switch (storage) {
+    case SVS_STORAGE_BF16:
+      return dispatch<__nv_bfloat16, __nv_bfloat16>(shape, op, grid, threads, L, descs, a, status, s, occ);
+    case SVS_STORAGE_F16: return dispatch<__half, __half>(shape, op, grid, threads, L, descs, a, status, s, occ);
+    case SVS_STORAGE_BF16_FLOW32:
+      return dispatch<float, __nv_bfloat16>(shape, op, grid, threads, L, descs, a, status, s, occ);
+    case SVS_STORAGE_F16_FLOW32: return dispatch<float, __half>(shape, op, grid, threads, L, descs, a, status, s, occ);
+    default: return dispatch<float, float>(shape, op, grid, threads, L, descs, a, status, s, occ);
+  }
+}
+
+}  // namespace svs

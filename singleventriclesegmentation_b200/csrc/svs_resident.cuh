@@ -1,0 +1,523 @@
+// The iterations of one warp with the whole state of a pair on chip.
+//
+// iterate_split_kernel reads and writes u, p, D, rho_c and the warped gradient through memory in
+// every iteration. Where a level's volume fits into the registers and shared memory of the GPU,
+// none of that traffic is needed: resident_kernel gives every CTA one box of a pair's volume and
+// runs all iterations of a warp (tvl13d.py:213-253) in one launch, p and the per-voxel constants
+// in registers, u and q = D p in shared memory. Only the faces of u and q cross CTAs.
+//
+// Per iteration and CTA:
+//   halo of u   the six faces of the neighbouring boxes' u arrive (below); barrier;
+//   dual        p_new = proj(p + sigma D grad u) of the own voxels, q = D p_new to shared memory,
+//               q_x / q_y / q_z of the box's faces published to the neighbours;
+//   halo of q   the neighbours' faces arrive; barrier;
+//   primal      u_new = prox(u - tau adjoint(q)) in place, faces of u published.
+// No dual is recomputed on a halo (the march kernels recompute 20-30%), and a thread owns NP
+// pairs of x-adjacent voxels (packed FP32 arithmetic) stacked along z, so the z neighbours of u
+// are mostly its own registers.
+//
+// Exchange: one 16-byte word per face voxel, {three components, tag}, written and polled with
+// single 128-bit relaxed accesses, so a word's data and its tag arrive together and no fence or
+// flag is needed. Each box has one incoming word per face voxel for u and one for q. A word is
+// overwritten only after it was read: a box publishes q(t+1) to a neighbour after consuming that
+// neighbour's u(t), which the neighbour published after consuming q(t); u likewise. Tags count
+// iterations from 1; the reader clears its words when the launch ends, so every launch starts
+// from tag 0. Polling is bounded (ResidentArgs::wait_us); a box that gives up raises the abort
+// word, which ends its neighbours' waits and the plan's later launches.
+//
+// Measured on one B200 (us per iteration; before: one launch per iteration, march along z):
+//   f16-flow32 80^3 10.6 (20.4), 48^3 3.4 (14.4), 40^3 3.3 (10.3), 20^3 2.8 (8.2);
+//   f32 48^3 3.4 (12.3), 20^3 2.8 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
+// Small boxes are bound by the two exchanges (about 2.5 us: publish, poll, barriers). 80^3 is
+// bound by the latency of 12 warps of 168 registers (about 8,000 cycles of dual, 5,800 of primal)
+// and by the words' L2 traffic (3.6 MB per exchange each way).
+//
+// Boundaries (MIRROR with power-of-two 0.5/h only, see resident_ok in svs_solver.cu): central
+// differences vanish on a face and the adjoint sees q = 0 there, so with u mirrored into the cell
+// outside the volume (u[-1] = u[1], u[n] = u[n-2]) and q's normal component zeroed on the face,
+// every voxel runs the interior stencil; 0.5/h being a power of two, the products are exact and
+// the difference is exactly zero. The arithmetic per voxel is that of iterate_split_kernel
+// (dual_row, primal_step, primal_apply, the same fused operations), so the results agree bitwise.
+#pragma once
+
+#include "svs_iterate.cuh"
+
+namespace svs {
+
+// A launch: up to kResSlots boxes of up to kResSlots pairs, as a kernel parameter (constant memory,
+// so that everything derived from it stays in uniform registers). Pair i's boxes are a
+// gx x gy x gz grid of bx x by x bz boxes (the last of an axis may reach past the volume), blocks
+// first .. first + gx gy gz - 1, x fastest; its neighbours are therefore at fixed distances.
+constexpr int kResSlots = 160;
+struct ResPair {
+  int desc, first;
+  unsigned char gx, gy, gz, pad0;
+  unsigned char bx, by, bz, pad1;
+};
+struct ResLaunch {
+  ResPair pair[kResSlots];
+  unsigned char of[kResSlots];  // pair of each block
+};
+
+struct ResidentArgs {
+  const float* sig;  // [iters] sigma and tau of each iteration
+  const float* tau;
+  float wm, wtv;     // weight_matching (factor = tau * wm), weight_tv
+  int src, dst;      // ping-pong copies read at the start and written at the end
+  int iters;
+  unsigned wait_us;  // bound of a wait for a neighbour
+  int words;         // exchange words per box and field
+  uint4* xbuf;       // [boxes][u, q][words]
+  int* abort;        // raised when a wait gave up
+};
+
+// Compiled shapes: NP voxel pairs per thread, up to NT threads; CU floats per component of u (with
+// its halo planes, rows and columns) and CQ of each of q_x (halo columns), q_y (halo rows) and
+// q_z (halo planes); up to NE face voxels per thread. KEEP_R: rho_c and the warped gradient stay
+// in registers (else they are read again in every iteration, before the wait for q's halo).
+template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_R_>
+struct ResShape {
+  static constexpr int NP = NP_, NT = NT_, CU = CU_, CQ = CQ_, NE = NE_;
+  static constexpr bool KEEP_R = KEEP_R_;
+  // the register file holds 16,384 registers per scheduler, a quarter of the warps each
+  static constexpr int WARPS = (NT + 31) / 32, MAXREG = 16384 / ((WARPS + 3) / 4 * 32) / 8 * 8;
+  static constexpr int REGS = MAXREG > 255 ? 255 : MAXREG;
+  static constexpr int SMEM = (3 * CU + 9 * CQ) * 4;
+  static_assert(SMEM <= 227 * 1024, "fits one CTA per SM");
+  static_assert(CU % 2 == 0 && CQ % 2 == 0, "8-byte aligned components");
+  static_assert(CU < 65536 && 7 * CQ < 65536, "cells are 16-bit");
+};
+
+// The state of a voxel pair in registers, as stored: float2, or two 16-bit values in one word.
+template <typename SP> struct Held;
+template <> struct Held<float> {
+  using T = float2;
+  static __device__ __forceinline__ void pin(float2&) {}
+  static __device__ __forceinline__ float2 get(float2 v) { return v; }
+  static __device__ __forceinline__ float2 put(float2 v) { return v; }
+};
+template <> struct Held<__half> {
+  using T = __half2;
+  static __device__ __forceinline__ void pin(__half2& v) { asm volatile("" : "+r"(reinterpret_cast<unsigned&>(v))); }
+  static __device__ __forceinline__ float2 get(__half2 v) { return __half22float2(v); }
+  static __device__ __forceinline__ __half2 put(float2 v) { return __floats2half2_rn(v.x, v.y); }
+};
+template <> struct Held<__nv_bfloat16> {
+  using T = __nv_bfloat162;
+  static __device__ __forceinline__ void pin(__nv_bfloat162& v) { asm volatile("" : "+r"(reinterpret_cast<unsigned&>(v))); }
+  static __device__ __forceinline__ float2 get(__nv_bfloat162 v) { return __bfloat1622float2(v); }
+  static __device__ __forceinline__ __nv_bfloat162 put(float2 v) { return __floats2bfloat162_rn(v.x, v.y); }
+};
+// u rounded to its storage type (the value the next iteration reads)
+template <typename SU> __device__ __forceinline__ float2 as_stored(float2 v) { return Held<SU>::get(Held<SU>::put(v)); }
+
+// Single 128-bit accesses at GPU scope: {a, b, c, tag}.
+__device__ __forceinline__ void word_publish(uint4* p, float a, float b, float c, unsigned tag) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
+      "mov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 t, {lo, hi};\n\t"
+      "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+      "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(__float_as_uint(c)), "r"(tag)
+      : "memory");
+}
+// ...read only if `on` (zeros otherwise: a word that is already here is not asked for again)
+__device__ __forceinline__ uint4 word_poll(const uint4* p, unsigned on) {
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\tmov.b64 lo, 0;\n\tmov.b64 hi, 0;\n\tmov.b128 t, {lo, hi};\n\t"
+      "@q ld.relaxed.gpu.global.b128 t, [%4];\n\tmov.b128 {lo, hi}, t;\n\t"
+      "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p), "r"(on)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return vadd(a, make_float2(-b.x, -b.y)); }
+
+template <typename SU, typename SP, typename C>
+__global__ void __launch_bounds__(C::NT) __maxnreg__(C::REGS)
+resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ descs, const ResidentArgs a,
+                int* __restrict__ status) {
+  constexpr int NP = C::NP;
+  using H = Held<SP>;
+  using HT = typename H::T;
+  extern __shared__ __align__(16) float sm[];
+  float* const su = sm;
+  float* const sqx = sm + 3 * C::CU;
+  float* const sqy = sqx + 3 * C::CQ;
+  float* const sqz = sqy + 3 * C::CQ;
+
+  const ResPair& B = L.pair[L.of[blockIdx.x]];
+  const Desc& d = descs[B.desc];
+  // a stopped pair (the flag is the same in every box of the pair), or an earlier launch gave up
+  if (__syncthreads_or((d.stop && *d.stop) || *reinterpret_cast<volatile int*>(a.abort))) return;
+  const int bx = __shfl_sync(~0u, (int)B.bx, 0), by = __shfl_sync(~0u, (int)B.by, 0), bz = __shfl_sync(~0u, (int)B.bz, 0);
+  const int box = blockIdx.x - B.first;
+  const int gz_ = box / (B.gx * B.gy), gy_ = (box - gz_ * B.gx * B.gy) / B.gx, gx_ = box - (gz_ * B.gy + gy_) * B.gx;
+  const int x0 = gx_ * bx, y0 = gy_ * by, z0 = gz_ * bz;
+  const int rx = d.nx - x0, ry = d.ny - y0, rz = d.nz - z0;  // voxels from the box's origin to the volume's end
+  const int bid = blockIdx.x, ny_step = B.gx, nz_step = B.gx * B.gy;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int PU = (by + 2) * bx, PX = by * bx;      // plane strides of u and q_y, of q_x and q_z
+  const int UXLO = (bz + 2) * PU, UXHI = UXLO + bz * by;  // halo columns, one cell per (z, y)
+  const int QXLO = bz * PX, QXHI = QXLO + bz * by;
+  const int nface = 2 * (bz * by + bz * bx + by * bx);
+  const int fy0 = 2 * bz * by, fz0 = fy0 + 2 * bz * bx;  // first y face word, first z face word
+  const int cs = (int)d.cs;
+  const int gplane = d.pitch * d.ny;
+  const SU* u_src = reinterpret_cast<const SU*>(d.u[a.src]);
+
+  for (int i = tid; i < C::SMEM / 4; i += nt) sm[i] = 0.f;
+  __syncthreads();
+
+  // ---- this thread's face voxels (word tid + i nt of each field): across a face with a neighbour,
+  // the own cell to publish and the halo cell to fill; on a face of the volume, the cell outside
+  // that mirrors u (filled from two cells further in) and the own cell whose q is zero
+  const int S = a.words;
+  unsigned ucell[C::NE], qcell[C::NE];  // halo | own << 16 (u's from 0, q's from sqx)
+  int word[C::NE];                      // word to publish to (u), -1: volume face, -2: none
+#pragma unroll
+  for (int i = 0; i < C::NE; ++i) {
+    const int e = tid + i * nt;
+    word[i] = -2;
+    ucell[i] = qcell[i] = 0;
+    if (e >= nface) continue;
+    int f, k, x = 0, y = 0, z = 0;
+    if (e < fy0) {
+      f = e >= bz * by;
+      k = e - f * bz * by;
+      z = k / by;
+      y = k - z * by;
+    } else if (e < fz0) {
+      f = 2 + (e - fy0 >= bz * bx);
+      k = e - fy0 - (f - 2) * bz * bx;
+      z = k / bx;
+      x = k - z * bx;
+    } else {
+      f = 4 + (e - fz0 >= by * bx);
+      k = e - fz0 - (f - 4) * by * bx;
+      y = k / bx;
+      x = k - y * bx;
+    }
+    if (x >= rx || y >= ry || z >= rz) continue;
+    const int ax = f >> 1, hi = f & 1;
+    const int n = ax == 0 ? bx : ax == 1 ? by : bz, r = ax == 0 ? rx : ax == 1 ? ry : rz;
+    const int org = ax == 0 ? x0 : ax == 1 ? y0 : z0, step = ax == 0 ? 1 : ax == 1 ? ny_step : nz_step;
+    const bool nb = hi ? r > n : org > 0;
+    const int m = min(n, r);  // the box's extent along the axis
+    auto at = [&](int v) {    // u cell at coordinate v along the axis (-1 and the box's end: halo)
+      const int cx = ax == 0 ? v : x, cy = ax == 1 ? v : y, cz = ax == 2 ? v : z;
+      if (cx < 0) return UXLO + cz * by + cy;
+      if (cx == bx) return UXHI + cz * by + cy;
+      return (cz + 1) * PU + (cy + 1) * bx + cx;
+    };
+    auto q_at = [&](int v) {  // cell of q's component normal to the face
+      if (ax == 0) return v < 0 ? QXLO + k : v == bx ? QXHI + k : (z * by + y) * bx + v;
+      if (ax == 1) return 3 * C::CQ + z * PU + (v + 1) * bx + x;
+      return 6 * C::CQ + (v + 1) * PX + k;
+    };
+    const int outside = hi ? m : -1, edge = hi ? m - 1 : 0;
+    if (nb) {
+      const int first = ax == 0 ? 0 : ax == 1 ? fy0 : fz0, other = first + (hi ? 0 : (fy0 * (ax == 0) + (fz0 - fy0) * (ax == 1) + (nface - fz0) * (ax == 2)) / 2);
+      word[i] = (bid + (hi ? step : -step)) * 2 * S + other + k;
+      ucell[i] = at(outside) | at(edge) << 16;
+      qcell[i] = q_at(outside) | q_at(edge) << 16;
+      const int vx = ax == 0 ? outside : x, vy = ax == 1 ? outside : y, vz = ax == 2 ? outside : z;
+      const int o = (z0 + vz) * gplane + (y0 + vy) * d.pitch + x0 + vx;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) su[c * C::CU + at(outside)] = Store<SU>::ld(u_src + (long long)c * cs + o);
+    } else {
+      word[i] = -1;
+      ucell[i] = at(outside) | at(hi ? m - 2 : 1) << 16;
+      qcell[i] = q_at(edge) << 16;
+    }
+  }
+
+  // ---- this thread's column: pairs (xl, xl+1) at (yl, zl0 .. zl0 + nj - 1)
+  const int hx = bx >> 1, ncol = hx * by;
+  const int zg = tid / ncol, col = tid - zg * ncol;
+  const int yl = col / hx, xl = 2 * (col - yl * hx), zl0 = zg * NP;
+  int nj = (xl < rx && yl < min(ry, by)) ? min(max(min(rz, bz) - zl0, 0), NP) : 0;
+  int iu = ((zl0 + 1) * (by + 2) + yl + 1) * bx + xl;  // own cell of u; of q_y: - PU
+  int iqx = (zl0 * by + yl) * bx + xl;                 // own cell of q_x; of q_z: + PX
+  // cells left and right of the pair (halo columns at the box's ends) and their step along z; of
+  // q_x: - dUQ at the ends
+  const bool xlo = xl == 0, xhi = xl + 2 == bx;
+  int aL = xlo ? UXLO + zl0 * by + yl : iu - 1, dL = xlo ? by : PU;
+  int aR = xhi ? UXHI + zl0 * by + yl : iu + 2, dR = xhi ? by : PU;
+  const int dUQ = UXLO - QXLO;
+  int o0 = (z0 + zl0) * gplane + (y0 + yl) * d.pitch + x0 + xl;
+
+  HT P[NP][9], D[NP][6], R[NP][4];
+  auto load_R = [&](int j) {
+    const int o = o0 + j * gplane;
+    R[j][0] = __ldg(reinterpret_cast<const HT*>(reinterpret_cast<const SP*>(d.rc) + o));
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      R[j][1 + c] = __ldg(reinterpret_cast<const HT*>(reinterpret_cast<const SP*>(d.gw) + (long long)c * cs + o));
+  };
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    const float2 zero = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < 9; ++c) P[j][c] = H::put(zero);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) D[j][c] = H::put(zero);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) R[j][c] = H::put(zero);
+    if (j < nj) {
+      const int o = o0 + j * gplane;
+      const bool two = xl + 1 < rx;
+      auto take = [&](const void* base, int c) {
+        HT v = *reinterpret_cast<const HT*>(reinterpret_cast<const SP*>(base) + (long long)c * cs + o);
+        if (!two) v = H::put(make_float2(H::get(v).x, 0.f));
+        return v;
+      };
+#pragma unroll
+      for (int c = 0; c < 9; ++c) P[j][c] = take(d.p[a.src], c);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) D[j][c] = take(d.D, c);
+      if constexpr (C::KEEP_R) load_R(j);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const SU* s = u_src + (long long)c * cs + o;
+        su[c * C::CU + iu + j * PU] = Store<SU>::ld(s);
+        if (two) su[c * C::CU + iu + j * PU + 1] = Store<SU>::ld(s + 1);
+      }
+    }
+  }
+
+  const float wtv2 = a.wtv * a.wtv;
+
+  auto pair_at = [](const float* p) { return *reinterpret_cast<const float2*>(p); };
+  const uint4* const in0 = a.xbuf + (long long)blockIdx.x * 2 * S;
+  const uint64_t wait_ns = (uint64_t)a.wait_us * 1000ull;
+  // faces of u (or of q) after every thread's part is in shared memory: published, or mirrored
+  // (zeroed) at the volume's faces
+  auto send = [&](bool q, unsigned tag) {
+    float* s = q ? sqx : su;
+    const int st = q ? C::CQ : C::CU;
+    float v[C::NE][3];
+#pragma unroll
+    for (int i = 0; i < C::NE; ++i) {  // (a thread without a voxel here reads cell 0)
+      const float* own = s + ((q ? qcell[i] : ucell[i]) >> 16);
+      v[i][0] = own[0];
+      v[i][1] = own[st];
+      v[i][2] = own[2 * st];
+    }
+#pragma unroll
+    for (int i = 0; i < C::NE; ++i) {
+      if (word[i] >= 0) {
+        word_publish(a.xbuf + word[i] + (q ? S : 0), v[i][0], v[i][1], v[i][2], tag);
+      } else if (word[i] == -1) {
+        float* out = s + (q ? qcell[i] >> 16 : ucell[i] & 0xffff);
+        out[0] = q ? 0.f : v[i][0];
+        out[st] = q ? 0.f : v[i][1];
+        out[2 * st] = q ? 0.f : v[i][2];
+      }
+    }
+  };
+  // waits for the neighbours' words of one field and stores them; false: gave up
+  auto receive = [&](bool q, unsigned tag) {
+    const uint4* in = in0 + (q ? S : 0);
+    float* s = q ? sqx : su;
+    const int st = q ? C::CQ : C::CU;
+    unsigned pending = 0;
+#pragma unroll
+    for (int i = 0; i < C::NE; ++i)
+      if (word[i] >= 0) pending |= 1u << i;
+    uint64_t t0 = 0;
+    for (unsigned spin = 0; pending; ++spin) {
+      uint4 w[C::NE];
+#pragma unroll
+      for (int i = 0; i < C::NE; ++i)
+        w[i] = word_poll(in + tid + i * nt, pending & (1u << i));
+#pragma unroll
+      for (int i = 0; i < C::NE; ++i) {
+        if (!(pending & (1u << i)) || w[i].w != tag) continue;
+        float* out = s + ((q ? qcell[i] : ucell[i]) & 0xffff);
+        out[0] = __uint_as_float(w[i].x);
+        out[st] = __uint_as_float(w[i].y);
+        out[2 * st] = __uint_as_float(w[i].z);
+        pending &= ~(1u << i);
+      }
+      if (pending && (spin & 31) == 31) {
+        if (*reinterpret_cast<volatile int*>(a.abort)) return false;
+        const uint64_t now = global_ns();
+        if (!t0) t0 = now;
+        else if (now - t0 > wait_ns) {
+          atomicExch(a.abort, 1);
+          return false;
+        }
+      }
+    }
+    return true;
+  };
+
+  // u mirrored outside the volume for the first iteration
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < C::NE; ++i)
+    if (word[i] == -1)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) su[c * C::CU + (ucell[i] & 0xffff)] = su[c * C::CU + (ucell[i] >> 16)];
+  __syncthreads();
+
+  bool bad = false;
+  float next_sigma = __ldg(a.sig), next_tau = __ldg(a.tau);
+  for (int it = 0; it < a.iters; ++it) {
+    // keeps what is derived from these from being computed once, before the loop, and held
+    asm volatile("" : "+r"(iu), "+r"(iqx), "+r"(aL), "+r"(aR), "+r"(dL), "+r"(dR), "+r"(o0), "+r"(nj));
+#pragma unroll
+    for (int j = 0; j < NP; ++j)
+#pragma unroll
+      for (int c = 0; c < 6; ++c) H::pin(D[j][c]);
+    const float sigma = next_sigma, tau = next_tau;
+    if (it + 1 < a.iters) {
+      next_sigma = __ldg(a.sig + it + 1);
+      next_tau = __ldg(a.tau + it + 1);
+    }
+    const float factor = __fmul_rn(tau, a.wm);  // opticalFlowOps.cu:440
+    const float hsigma = 0.5f * sigma;
+    // ---- dual
+    if (nj > 0) {
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+        if (j < nj) {
+          const int i = iu + j * PU;
+          // every read of u before the first write of q (the compiler cannot tell them apart)
+          float2 e[3][3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const float* s = su + c * C::CU;
+            const float2 o = pair_at(s + i);
+            e[c][0] = vsub(make_float2(o.y, s[aR + j * dR]), make_float2(s[aL + j * dL], o.x));
+            e[c][1] = vsub(pair_at(s + i + bx), pair_at(s + i - bx));
+            e[c][2] = vsub(pair_at(s + i + PU), pair_at(s + i - PU));
+          }
+          float2 Dk[6];
+#pragma unroll
+          for (int c = 0; c < 6; ++c) Dk[c] = H::get(D[j][c]);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            float2 p0 = H::get(P[j][3 * c]), p1 = H::get(P[j][3 * c + 1]), p2 = H::get(P[j][3 * c + 2]);
+            dual_row(Dk, e[c][0], e[c][1], e[c][2], p0, p1, p2, hsigma, a.wtv, wtv2);
+            *reinterpret_cast<float2*>(sqx + c * C::CQ + iqx + j * PX) = dot3(Dk[0], Dk[1], Dk[2], p0, p1, p2);
+            *reinterpret_cast<float2*>(sqy + c * C::CQ + i - PU) = dot3(Dk[1], Dk[3], Dk[4], p0, p1, p2);
+            *reinterpret_cast<float2*>(sqz + c * C::CQ + iqx + PX + j * PX) = dot3(Dk[2], Dk[4], Dk[5], p0, p1, p2);
+            P[j][3 * c] = H::put(p0);
+            P[j][3 * c + 1] = H::put(p1);
+            P[j][3 * c + 2] = H::put(p2);
+          }
+        }
+      }
+    }
+    if constexpr (!C::KEEP_R) {
+#pragma unroll
+      for (int j = 0; j < NP; ++j)
+        if (j < nj) load_R(j);
+    }
+    __syncthreads();
+    send(true, (unsigned)it + 1);
+    bad = !receive(true, (unsigned)it + 1);
+    if (__syncthreads_or(bad)) {
+      bad = true;
+      break;
+    }
+    // ---- primal
+    asm volatile("" : "+r"(iu), "+r"(iqx), "+r"(aL), "+r"(aR));
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      if (j < nj) {
+        float2 uo[3], g[3], n[3], dv[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          uo[c] = pair_at(su + c * C::CU + iu + j * PU);
+          g[c] = H::get(R[j][1 + c]);
+        }
+        const float2 t = primal_step(uo, factor, H::get(R[j][0]), g);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float* qx = sqx + c * C::CQ;
+          const float* qy = sqy + c * C::CQ + iu - PU + j * PU;
+          const float* qz = sqz + c * C::CQ + iqx + PX + j * PX;
+          const float2 o = pair_at(qx + iqx + j * PX);
+          const float2 dx = vsub(make_float2(qx[xlo ? aL - dUQ + j * by : iqx + j * PX - 1], o.x),
+                                 make_float2(o.y, qx[xhi ? aR - dUQ + j * by : iqx + j * PX + 2]));
+          const float2 dy = vsub(pair_at(qy - bx), pair_at(qy + bx));
+          const float2 dz = vsub(pair_at(qz - PX), pair_at(qz + PX));
+          dv[c] = sum3(dx, dy, dz);
+        }
+        primal_apply(uo, dv, 0.5f * tau, t, g, n);
+        // (the voxel beside the volume's last one, odd nx: a mirror cell, filled again below)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          *reinterpret_cast<float2*>(su + c * C::CU + iu + j * PU) = as_stored<SU>(n[c]);
+      }
+    }
+    if (it + 1 < a.iters) {
+      __syncthreads();
+      send(false, (unsigned)it + 1);
+      bad = !receive(false, (unsigned)it + 1);
+      if (__syncthreads_or(bad)) {
+        bad = true;
+        break;
+      }
+    }
+  }
+  if (bad) {
+    if (tid == 0) atomicOr(status, SVS_DEV_TIMEOUT);
+    return;
+  }
+
+  // ---- state back to memory, incoming words cleared for the next launch. The neighbours read
+  // their first halos from copy `src` before they published what this box consumed, so the write
+  // may go to the same copy.
+  SU* u_dst = reinterpret_cast<SU*>(d.u[a.dst]);
+  SP* p_dst = reinterpret_cast<SP*>(d.p[a.dst]);
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    if (j < nj) {
+      const int o = o0 + j * gplane;
+      const bool two = xl + 1 < rx;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float2 v = pair_at(su + c * C::CU + iu + j * PU);
+        SU* s = u_dst + (long long)c * cs + o;
+        Store<SU>::st(s, v.x);
+        if (two) Store<SU>::st(s + 1, v.y);
+      }
+#pragma unroll
+      for (int c = 0; c < 9; ++c) {
+        SP* s = p_dst + (long long)c * cs + o;
+        if (two) *reinterpret_cast<HT*>(s) = P[j][c];
+        else Store<SP>::st(s, H::get(P[j][c]).x);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < C::NE; ++i) {
+    if (word[i] < 0) continue;
+    word_publish(const_cast<uint4*>(in0) + tid + i * nt, 0.f, 0.f, 0.f, 0u);
+    word_publish(const_cast<uint4*>(in0) + S + tid + i * nt, 0.f, 0.f, 0.f, 0u);
+  }
+}
+
+// Compiled shapes, every storage mode (svs_resident.cu).
+using ResSmall = ResShape<1, 512, 1920, 1408, 4, true>;
+using ResMid = ResShape<2, 512, 3456, 2688, 4, false>;
+using ResLarge = ResShape<5, 384, 5408, 4480, 4, false>;
+constexpr int kResShapes = 3, kResMaxWords = 2048;
+// Host view of a shape: voxel pairs and threads, floats per component, face words per thread.
+struct ResCaps {
+  int np, nt, cu, cq, ne;
+};
+template <typename C> constexpr ResCaps res_caps() { return {C::NP, C::NT, C::CU, C::CQ, C::NE}; }
+constexpr ResCaps kResCaps[kResShapes] = {res_caps<ResSmall>(), res_caps<ResMid>(), res_caps<ResLarge>()};
+
+// op 0: set the kernel's shared-memory attribute and return the CTAs one SM holds in *occ (false:
+// not usable); op 1: one cooperative launch of `grid` CTAs of `threads` threads on stream s.
+bool resident_variant(int storage, int shape, int op, unsigned grid, unsigned threads, const ResLaunch* L,
+                      const Desc* descs, const ResidentArgs* a, int* status, cudaStream_t s, int* occ);
+
+}  // namespace svs

@@ -32,6 +32,7 @@
 
 #include "svs_common.cuh"
 #include "svs_iterate.cuh"
+#include "svs_resident.cuh"
 
 namespace svs {
 namespace {
@@ -601,6 +602,18 @@ struct svs_plan {
   float* d_sig = nullptr;                  // [max_outer_iterations] schedule on the device
   float* d_tau = nullptr;
   unsigned* d_gridbar = nullptr;           // grid-barrier arrival counter
+  // resident iterations (svs_resident.cuh): per level, the launches that cover resident[level]'s
+  // pairs; the other pairs of the level run the per-iteration kernels
+  struct ResStep {
+    int shape = 0, words = 0;
+    unsigned grid = 0, threads = 0;
+    svs::ResLaunch launch;
+  };
+  std::vector<std::vector<ResStep>> res_steps;  // [level]
+  std::vector<std::vector<char>> resident;      // [level][pair]
+  bool no_resident = false;                // the launches could not be captured here
+  uint4* d_xbuf = nullptr;                 // exchange words, then the abort word
+  size_t xbuf_bytes = 0;
 };
 
 namespace svs {
@@ -823,19 +836,23 @@ int auto_choice(int storage, int n, const int* dims, int sms, int* pair_tid) {
   return main_tid;
 }
 
+// (the pairs in P.pair_mask when set)
 int auto_level(const svs_plan& P, int level, std::vector<int>& pair_tid) {
-  std::vector<int> dims(3 * (size_t)P.num_pairs);
+  std::vector<int> dims, members, tids;
   for (int i = 0; i < P.num_pairs; ++i) {
+    if (P.pair_mask && !(*P.pair_mask)[i]) continue;
     const Desc& d = P.h_descs[(size_t)level * P.num_pairs + i];
-    dims[3 * i] = d.nz;
-    dims[3 * i + 1] = d.ny;
-    dims[3 * i + 2] = d.nx;
+    members.push_back(i);
+    dims.insert(dims.end(), {d.nz, d.ny, d.nx});
   }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   pair_tid.assign(P.num_pairs, 0);
-  return auto_choice(P.prm.storage, P.num_pairs, dims.data(), sms, pair_tid.data());
+  tids.assign(members.size(), 0);
+  const int tid = auto_choice(P.prm.storage, (int)members.size(), dims.data(), sms, tids.data());
+  for (size_t k = 0; k < members.size(); ++k) pair_tid[members[k]] = tids[k];
+  return tid;
 }
 
 // z chunks per column for a split-role variant. The launch's CTAs are dispatched in tile-list
@@ -944,6 +961,255 @@ void build_tiles(svs_plan& P, int level, int tid, std::vector<Tile>* out_opt = n
   out.insert(out.end(), tail.begin(), tail.end());
 }
 
+// Work that holds resident launches takes turns on a device: their CTAs wait for one another, so
+// two such launches from two streams must not each hold a part of the SMs. (A cooperative launch
+// starts only as a whole; this does not lean on two of them never interleaving.) The constructor
+// makes the stream wait for the previous turn, the destructor ends this one. A stream under
+// capture takes none: events cannot cross into a capture.
+class ResidentTurn {
+ public:
+  explicit ResidentTurn(cudaStream_t s, bool on = true) : s_(s) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (!on || cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= kDevices ||
+        cudaStreamIsCapturing(s, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone)
+      return;
+    lock_ = std::unique_lock<std::mutex>(mutex());
+    cudaEvent_t& e = event(dev_);
+    if (e && cudaStreamWaitEvent(s, e, 0) != cudaSuccess) {  // the device was reset
+      cudaGetLastError();
+      e = nullptr;
+    }
+    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      e = nullptr;
+    }
+  }
+  ~ResidentTurn() {
+    if (lock_.owns_lock() && event(dev_)) cudaEventRecord(event(dev_), s_);
+  }
+
+ private:
+  static constexpr int kDevices = 64;
+  static std::mutex& mutex() {
+    static std::mutex m;
+    return m;
+  }
+  static cudaEvent_t& event(int dev) {
+    static cudaEvent_t e[kDevices] = {};
+    return e[dev];
+  }
+  cudaStream_t s_;
+  int dev_ = 0;
+  std::unique_lock<std::mutex> lock_;
+};
+
+// Modelled microseconds per iteration, fitted to measurements on one B200.
+// The per-iteration kernels over a level's voxels (2-byte fields, 80^3 pairs: 20.3 us for one, 54
+// for 4, 142 for 12, 670 for 68; f32: 20.5 for one, 72 for 4): launch and ramp, bandwidth, and the
+// unfilled last wave of a small batch.
+double stream_us(int storage, double voxels) {
+  if (voxels <= 0.0) return 0.0;
+  return 10.0 + voxels * (storage == SVS_STORAGE_F32 ? 28e-6 : 19.3e-6) + std::min(14.0, 1.6e-6 * voxels);
+}
+// A resident launch with boxes of `threads` threads of `np` voxel pairs and `words` face words:
+// the two exchanges (2.5 us with next to no work), the warps' pairs, the words' traffic. 6x6x6
+// boxes 2.7 us, 8x8x10 3.4, 10x10x10 4.1 (np 1), 20x8x8 4.6, 20x10x10 6.1 (np 2; f32 5.3 and 6.9),
+// 16x12x20 10.6 (np 5).
+float resident_us(int storage, int np, int threads, int words) {
+  const float pair_us = np > 2 ? 0.12f : np == 2 && storage == SVS_STORAGE_F32 ? 0.11f : 0.085f;
+  return 2.45f + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words;
+}
+
+// ---- resident iterations (svs_resident.cuh): which pairs of a level, in which boxes
+struct ResBoxes {
+  int bx, by, bz, threads, words;
+  float us;  // modelled time per iteration
+};
+// Boxes that fit a compiled shape, by modelled time: x in pairs, z in whole groups of NP pairs.
+std::vector<ResBoxes> resident_boxes(int storage, const ResCaps& c) {
+  std::vector<ResBoxes> out;
+  for (int bx = 4; bx <= 64; bx += 2)
+    for (int by = 2; by <= 48; ++by)
+      for (int bz = std::max(2, c.np); bz <= 48; bz += c.np) {
+        const int threads = bx / 2 * by * (bz / c.np);
+        const int words = 2 * (bz * by + bz * bx + by * bx);
+        if (threads > c.nt) break;
+        if (words > c.ne * (int)ceil_div(threads, 32) * 32) continue;
+        const int col = 2 * bz * by;
+        if ((bz + 2) * (by + 2) * bx + col > c.cu || std::max(bz * by * bx + col, std::max(bz * (by + 2) * bx, (bz + 2) * by * bx)) > c.cq)
+          continue;
+        out.push_back({bx, by, bz, threads, words, resident_us(storage, c.np, threads, words)});
+      }
+  std::sort(out.begin(), out.end(), [](const ResBoxes& a, const ResBoxes& b) { return a.us < b.us; });
+  return out;
+}
+// Boxes of a volume with no box one voxel thick at its end (the mirrored cell and its source lie
+// in one box), 0 if that fails.
+int resident_count(const Desc& d, const ResBoxes& b) {
+  if (d.nx % b.bx == 1 || d.ny % b.by == 1 || d.nz % b.bz == 1) return 0;
+  return (int)(ceil_div(d.nx, b.bx) * ceil_div(d.ny, b.by) * ceil_div(d.nz, b.bz));
+}
+// The stencils of resident_kernel: MIRROR, unit spacing, at least 4 nodes per axis.
+bool resident_ok(const svs_plan& P, const Desc& d) {
+  return P.prm.boundary == SVS_BOUNDARY_MIRROR && d.hx == 1.f && d.hy == 1.f && d.hz == 1.f && d.nx >= 4 &&
+         d.ny >= 4 && d.nz >= 4;
+}
+
+// Fills P.resident[level] and P.res_steps[level]. For each compiled shape and each bound on the
+// modelled time of a box, every pair takes the fewest boxes within the bound and the pairs are
+// packed into launches of at most one box per SM; the packing with the least total time is
+// taken if it beats the per-iteration kernels.
+void plan_resident(svs_plan& P, int level) {
+  const int np = P.num_pairs;
+  P.resident[level].assign(np, 0);
+  P.res_steps[level].clear();
+  const bool req = P.tile_id > 0 || (level < (int)P.level_tile_req.size() && P.level_tile_req[level] > 0) ||
+                   (level < (int)P.level_chunks_req.size() && P.level_chunks_req[level] > 0) ||
+                   (level < (int)P.pair_tile_req.size() &&
+                    std::any_of(P.pair_tile_req[level].begin(), P.pair_tile_req[level].end(), [](int t) { return t > 0; }));
+  if (req || P.persistent || P.no_resident || P.stall_level == level || P.prm.max_outer_iterations < 2) return;
+  int dev = 0, sms = 148, coop = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  if (!coop) return;
+  const int slots = std::min(sms, kResSlots);
+  const Desc* D = P.h_descs.data() + (size_t)level * np;
+  struct Choice {
+    float us;
+    int count, box;
+  };
+  double best_us = -1.0, all_vox = 0.0;
+  int best_shape = -1;
+  std::vector<int> best_box;
+  std::vector<std::vector<ResBoxes>> boxes(kResShapes);
+  for (int i = 0; i < np; ++i) all_vox += (double)D[i].n;
+  for (int sh = 0; sh < kResShapes; ++sh) {
+    int occ = 0;
+    if (!resident_variant(P.prm.storage, sh, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, &occ)) continue;
+    boxes[sh] = resident_boxes(P.prm.storage, kResCaps[sh]);
+    // per pair: fewer boxes for more time
+    std::vector<std::vector<Choice>> front(np);
+    std::vector<float> bounds;
+    double vox = 0.0;
+    for (int i = 0; i < np; ++i) {
+      if (!resident_ok(P, D[i])) continue;
+      int same = -1;
+      for (int k = 0; k < i && same < 0; ++k)
+        if (D[k].nx == D[i].nx && D[k].ny == D[i].ny && D[k].nz == D[i].nz) same = k;
+      if (same >= 0) {
+        front[i] = front[same];
+      } else {
+        int fewest = slots + 1;
+        for (int b = 0; b < (int)boxes[sh].size(); ++b) {
+          const int n = resident_count(D[i], boxes[sh][b]);
+          if (n <= 0 || n >= fewest) continue;
+          fewest = n;
+          front[i].push_back({boxes[sh][b].us, n, b});
+          bounds.push_back(boxes[sh][b].us);
+        }
+      }
+      if (!front[i].empty()) vox += (double)D[i].n;
+    }
+    std::sort(bounds.begin(), bounds.end());
+    bounds.erase(std::unique(bounds.begin(), bounds.end()), bounds.end());
+    for (const float bound : bounds) {
+      std::vector<int> pick(np, -1);
+      double total = 0.0;
+      float longest = 0.f;
+      int used = 0;
+      bool ok = true;
+      for (int i = 0; i < np && ok; ++i) {
+        if (front[i].empty()) continue;
+        const Choice* c = nullptr;
+        for (const Choice& q : front[i])
+          if (q.us <= bound) c = &q;
+        if (!c) { ok = false; break; }
+        pick[i] = c->box;
+        if (used + c->count > slots) {
+          total += longest;
+          used = 0;
+          longest = 0.f;
+        }
+        used += c->count;
+        longest = std::max(longest, c->us);
+      }
+      total += longest;
+      // the pairs left out keep the per-iteration launches
+      if (!ok || vox == 0.0) continue;
+      total += stream_us(P.prm.storage, all_vox - vox);
+      if (best_us < 0 || total < best_us) {
+        best_us = total;
+        best_shape = sh;
+        best_box = pick;
+      }
+    }
+  }
+  if (best_us < 0 || best_us >= stream_us(P.prm.storage, all_vox)) return;
+  svs_plan::ResStep st;
+  int npairs = 0;
+  auto flush = [&] {
+    if (npairs) P.res_steps[level].push_back(st);
+    st = svs_plan::ResStep{};
+    npairs = 0;
+  };
+  for (int i = 0; i < np; ++i) {
+    if (best_box[i] < 0) continue;
+    const ResBoxes& b = boxes[best_shape][best_box[i]];
+    const int n = resident_count(D[i], b);
+    if (st.grid + n > (unsigned)slots) flush();
+    ResPair& r = st.launch.pair[npairs];
+    r.desc = level * np + i;
+    r.first = (int)st.grid;
+    r.gx = (unsigned char)ceil_div(D[i].nx, b.bx);
+    r.gy = (unsigned char)ceil_div(D[i].ny, b.by);
+    r.gz = (unsigned char)ceil_div(D[i].nz, b.bz);
+    r.bx = (unsigned char)b.bx;
+    r.by = (unsigned char)b.by;
+    r.bz = (unsigned char)b.bz;
+    for (int k = 0; k < n; ++k) st.launch.of[st.grid + k] = (unsigned char)npairs;
+    st.shape = best_shape;
+    st.grid += (unsigned)n;
+    st.threads = std::max(st.threads, (unsigned)ceil_div(b.threads, 32) * 32);
+    st.words = std::max(st.words, b.words);
+    ++npairs;
+    P.resident[level][i] = 1;
+  }
+  flush();
+}
+
+bool any_resident(const svs_plan& P) {
+  for (const auto& l : P.res_steps)
+    if (!l.empty()) return true;
+  return false;
+}
+bool all_resident(const svs_plan& P, int level) {
+  return level < (int)P.resident.size() && !P.resident[level].empty() &&
+         std::all_of(P.resident[level].begin(), P.resident[level].end(), [](char c) { return c != 0; });
+}
+
+// `iters` iterations of the level's resident pairs, from ping-pong copy `cur` to cur ^ (iters & 1).
+// Returns the launches issued, -1 after a launch error.
+int resident_iterations(svs_plan& P, int level, int iters, int cur, cudaStream_t s) {
+  for (const svs_plan::ResStep& st : P.res_steps[level]) {
+    ResidentArgs a;
+    a.sig = P.d_sig;
+    a.tau = P.d_tau;
+    a.wm = P.prm.weight_matching;
+    a.wtv = P.prm.weight_tv;
+    a.src = cur;
+    a.dst = cur ^ (iters & 1);
+    a.iters = iters;
+    a.wait_us = P.wait_us;
+    a.words = st.words;
+    a.xbuf = P.d_xbuf;
+    a.abort = reinterpret_cast<int*>(reinterpret_cast<char*>(P.d_xbuf) + P.xbuf_bytes - 256);
+    if (!resident_variant(P.prm.storage, st.shape, 1, st.grid, st.threads, &st.launch, P.d_descs, &a, P.d_status, s, nullptr))
+      return -1;
+  }
+  return (int)P.res_steps[level].size();
+}
+
 // (Re)build tile lists and TMA descriptors for the requested tile id.
 svs_status setup_tiles(svs_plan& P) {
   const int want = P.tile_id;
@@ -955,10 +1221,20 @@ svs_status setup_tiles(svs_plan& P) {
   P.extra.assign(P.levels, {});
   std::vector<TMaps> maps((size_t)P.levels * P.num_pairs);
   std::memset(maps.data(), 0, maps.size() * sizeof(TMaps));
+  P.res_steps.assign(P.levels, {});
+  P.resident.assign(P.levels, {});
   for (int l = 0; l < P.levels; ++l) {
+    plan_resident(P, l);
+    // per-iteration lists: the pairs that are not resident (all of them where every pair is, for
+    // the queries and as what a tile request starts from)
+    std::vector<char> rest(P.num_pairs, 1);
+    if (!all_resident(P, l))
+      for (int i = 0; i < P.num_pairs; ++i) rest[i] = !P.resident[l][i];
     const int req = (l < (int)P.level_tile_req.size() && P.level_tile_req[l] > 0) ? P.level_tile_req[l] : want;
     std::vector<int> autop;
+    P.pair_mask = &rest;
     int tid = req > 0 ? req : auto_level(P, l, autop);
+    P.pair_mask = nullptr;
     // per-pair requests (and, without a level request, the automatic per-pair choices) that
     // differ from the level's variant form groups of their own
     std::vector<int> own(P.num_pairs, 0);
@@ -971,7 +1247,7 @@ svs_status setup_tiles(svs_plan& P) {
       for (const AutoCost& c : kAutoCosts16) {
         std::vector<char> gm(P.num_pairs, 0);
         bool any = false;
-        for (int i = 0; i < P.num_pairs; ++i) any |= gm[i] = !own[i] && autop[i] == c.tid;
+        for (int i = 0; i < P.num_pairs; ++i) any |= gm[i] = rest[i] && !own[i] && autop[i] == c.tid;
         if (!any) continue;
         P.pair_mask = &gm;
         usable = usable && iter_dispatch(P, &maps, l, c.tid, 0, nullptr, nullptr);
@@ -981,7 +1257,7 @@ svs_status setup_tiles(svs_plan& P) {
         if (!own[i]) own[i] = autop[i];
     }
     std::vector<char> mask(P.num_pairs, 1);
-    for (int i = 0; i < P.num_pairs; ++i) mask[i] = own[i] == 0 || own[i] == tid;
+    for (int i = 0; i < P.num_pairs; ++i) mask[i] = rest[i] && (own[i] == 0 || own[i] == tid);
     P.pair_mask = &mask;
     // attributes and tensor maps first: the tile builder asks the occupancy calculator
     if (!iter_dispatch(P, &maps, l, tid, 0, nullptr, nullptr)) {
@@ -990,18 +1266,18 @@ svs_status setup_tiles(svs_plan& P) {
         return fail(SVS_ERR_UNSUPPORTED, "tile variant not usable for this plan (shared memory or TMA descriptor limits)");
       }
       tid = 6;  // plain-load 32x8
-      for (int i = 0; i < P.num_pairs; ++i) mask[i] = own[i] == 0 || own[i] == tid;
+      for (int i = 0; i < P.num_pairs; ++i) mask[i] = rest[i] && (own[i] == 0 || own[i] == tid);
     }
     build_tiles(P, l, tid);
     P.level_tile[l] = tid;
     for (int i = 0; i < P.num_pairs; ++i) {
-      if (mask[i]) continue;
+      if (mask[i] || !rest[i]) continue;
       const int g = own[i];
       bool seen = false;
       for (auto& grp : P.extra[l]) seen |= grp.tid == g;
       if (seen) continue;
       std::vector<char> gm(P.num_pairs, 0);
-      for (int j = 0; j < P.num_pairs; ++j) gm[j] = own[j] == g && !mask[j];
+      for (int j = 0; j < P.num_pairs; ++j) gm[j] = rest[j] && own[j] == g && !mask[j];
       P.pair_mask = &gm;
       if (!iter_dispatch(P, &maps, l, g, 0, nullptr, nullptr)) {
         P.pair_mask = nullptr;
@@ -1015,7 +1291,7 @@ svs_status setup_tiles(svs_plan& P) {
     P.pair_mask = nullptr;
     P.pair_used[l].assign(P.num_pairs, tid);
     for (int i = 0; i < P.num_pairs; ++i)
-      if (!mask[i]) P.pair_used[l][i] = own[i];
+      if (!mask[i] && rest[i]) P.pair_used[l][i] = own[i];
   }
   // persistent iteration loop: levels whose pairs share one split-role variant that has the form
   P.level_persist.assign(P.levels, 0);
@@ -1051,6 +1327,12 @@ svs_status setup_tiles(svs_plan& P) {
     svs_status st = check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "group event");
     if (st) return st;
     P.events.push_back(e);
+  }
+  if (any_resident(P) && !P.d_xbuf) {
+    P.xbuf_bytes = (size_t)kResSlots * 2 * kResMaxWords * sizeof(uint4) + 256;
+    svs_status st = check_cuda(cudaMalloc((void**)&P.d_xbuf, P.xbuf_bytes), "exchange words");
+    if (!st) st = check_cuda(cudaMemset(P.d_xbuf, 0, P.xbuf_bytes), "exchange words");
+    if (st) return st;
   }
   return check_cuda(cudaMemcpy(P.d_maps, maps.data(), maps.size() * sizeof(TMaps), cudaMemcpyHostToDevice), "tensor maps");
 }
@@ -1137,6 +1419,9 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
   long long launches = 0;
   auto grid = [&](int level) { return dim3(ceil_div(max_voxels(P, level), 256), np); };
   const Desc* D = P.d_descs;
+  // exchange words of the resident launches start from tag 0 (each launch leaves them so, unless
+  // a wait gave up)
+  if (any_resident(P)) cudaMemsetAsync(P.d_xbuf, 0, P.xbuf_bytes, s);
   blur_pair_kernel<<<grid(0), 256, 0, s>>>(D, P.d_raw, P.blur_r, P.blur, q.use_gaussian_blur);
   ++launches;
   for (int l = 1; l < L; ++l) {
@@ -1182,6 +1467,14 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
         ++launches;
         cur ^= q.max_outer_iterations & 1;
       } else {
+        if (l < (int)P.res_steps.size() && !P.res_steps[l].empty()) {
+          const int n = resident_iterations(P, l, q.max_outer_iterations, cur, s);
+          if (n < 0) return -1;
+          launches += n;
+        }
+        if (all_resident(P, l)) {
+          cur ^= q.max_outer_iterations & 1;
+        } else {
         fork_groups(P, l, s);
         for (int it = 0; it < q.max_outer_iterations; ++it) {
           const IterArgs a = iter_args(P, it, cur);
@@ -1189,6 +1482,7 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
           cur ^= 1;
         }
         join_groups(P, l, s);
+        }
       }
       if (P.res_on) {
         residual_kernel<SU><<<grid(l), 256, 0, s>>>(D + (size_t)l * np, cur, P.d_snaps, P.d_acc, 0);
@@ -1455,7 +1749,7 @@ svs_status svs_tvl1_plan_destroy(svs_plan* P) {
   cudaFree(P->d_descs); cudaFree(P->d_raw); cudaFree(P->d_uout); cudaFree(P->d_umed);
   cudaFree(P->d_pout); cudaFree(P->d_uinit); cudaFree(P->d_pinit); cudaFree(P->d_maps);
   cudaFree(P->d_status);
-  cudaFree(P->d_sig); cudaFree(P->d_tau); cudaFree(P->d_gridbar);
+  cudaFree(P->d_sig); cudaFree(P->d_tau); cudaFree(P->d_gridbar); cudaFree(P->d_xbuf);
   for (auto& lv : P->extra)
     for (auto& grp : lv) cudaFree(grp.d);
   for (cudaStream_t st_ : P->side) cudaStreamDestroy(st_);
@@ -1602,13 +1896,14 @@ svs_status svs_tvl1_solve_batch(svs_plan* P, const svs_pair_desc* pairs, int num
     if (st) return st;
     long long nl = enqueue(*P, P->cap_stream);
     cudaError_t ce = cudaStreamEndCapture(P->cap_stream, &g);
-    if ((nl < 0 || ce != cudaSuccess) && P->persistent) {
-      // the cooperative launch of the persistent loop could not be captured here: per-iteration
-      // launches instead (svs_tvl1_plan_level_persistent then reports 0)
+    if ((nl < 0 || ce != cudaSuccess) && (P->persistent || any_resident(*P))) {
+      // the cooperative launches of the persistent loop or the resident iterations could not be
+      // captured here: per-iteration launches instead (svs_tvl1_plan_level_persistent reports 0)
       if (g) cudaGraphDestroy(g);
       g = nullptr;
       cudaGetLastError();
       P->persistent = false;
+      P->no_resident = true;
       st = setup_tiles(*P);
       if (st) return st;
       st = check_cuda(cudaStreamBeginCapture(P->cap_stream, cudaStreamCaptureModeThreadLocal), "solve: capture");
@@ -1627,7 +1922,10 @@ svs_status svs_tvl1_solve_batch(svs_plan* P, const svs_pair_desc* pairs, int num
     P->graph_warm = warm;
     P->graph_want_p = want_p;
   }
-  st = check_cuda(cudaGraphLaunch(P->exec, s), "solve: graph launch");
+  {
+    ResidentTurn turn(any_resident(*P) ? s : nullptr, any_resident(*P));
+    st = check_cuda(cudaGraphLaunch(P->exec, s), "solve: graph launch");
+  }
   if (st) return st;
   count_launches(P->graph_kernels);
   for (int i = 0; i < num_pairs && !st; ++i) {
@@ -1650,6 +1948,19 @@ svs_status svs_tvl1_bench_iterations(svs_plan* P, int level, int count, svs_stre
   }
   int cur = 0;
   uint64_t launches = 0;
+  if (!P->res_steps[level].empty()) {
+    ResidentTurn turn(stream);
+    cudaMemsetAsync(P->d_xbuf, 0, P->xbuf_bytes, stream);
+    for (int done = 0; done < count; done += P->prm.max_outer_iterations) {
+      const int n = std::min(count - done, P->prm.max_outer_iterations);
+      const int k = resident_iterations(*P, level, n, cur, stream);
+      if (k < 0) return fail(SVS_ERR_LAUNCH, std::string("svs_tvl1_bench_iterations: ") + cudaGetErrorString(cudaGetLastError()));
+      launches += (uint64_t)k;
+      cur ^= n & 1;
+    }
+    if (all_resident(*P, level)) return check_launch("svs_tvl1_bench_iterations", launches);
+    cur = 0;
+  }
   fork_groups(*P, level, stream);
   for (int i = 0; i < count; ++i) {
     const int it = P->prm.max_outer_iterations > 0 ? i % P->prm.max_outer_iterations : 0;
@@ -1698,6 +2009,11 @@ int64_t svs_tvl1_plan_level_ctas(const svs_plan* P, int level) {
   if (level < (int)P->extra.size())
     for (const auto& grp : P->extra[level]) n += (int64_t)grp.h.size();
   return n;
+}
+
+int svs_tvl1_plan_level_resident(const svs_plan* P, int level) {
+  if (!P || level < 0 || level >= (int)P->resident.size()) return 0;
+  return (int)std::count(P->resident[level].begin(), P->resident[level].end(), (char)1);
 }
 
 svs_status svs_tvl1_plan_check(svs_plan* P) {

@@ -122,8 +122,12 @@ class SolverPlan:
         """Variant each pair runs at `level` (its group's or the level's; after a solve)."""
         return [int(_lib.lib().svs_tvl1_plan_pair_tile_used(self._h, int(level), i)) for i in range(len(self.dims))]
 
+    def level_resident(self, level: int) -> int:
+        """Pairs of `level` whose iterations run on chip, all of a warp in one launch (after a solve)."""
+        return int(_lib.lib().svs_tvl1_plan_level_resident(self._h, int(level)))
+
     def level_ctas(self, level: int) -> int:
-        """CTAs of one iterate launch at `level` (all variant groups; 0 before the first solve)."""
+        """CTAs of one per-iteration launch at `level` (all variant groups; 0 before the first solve)."""
         return int(_lib.lib().svs_tvl1_plan_level_ctas(self._h, int(level)))
 
     def set_level_chunks(self, level: int, chunks: int) -> None:
