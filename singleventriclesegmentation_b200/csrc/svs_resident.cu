@@ -36,9 +36,7 @@ bool dispatch(int shape, int op, unsigned grid, unsigned threads, const ResLaunc
   switch (shape) {
     case 0: return run<SU, SP, ResSmall>(op, grid, threads, L, descs, a, status, s, occ);
     case 1: return run<SU, SP, ResMid>(op, grid, threads, L, descs, a, status, s, occ);
-    case 2:
-      if constexpr (sizeof(SP) == 2) return run<SU, SP, ResLarge>(op, grid, threads, L, descs, a, status, s, occ);
-      return false;
+    case 2: return run<SU, SP, ResLarge<SP>>(op, grid, threads, L, descs, a, status, s, occ);
     default: return false;
   }
 }

@@ -27,10 +27,12 @@
 //
 // Measured on one B200 (us per iteration; before: one launch per iteration, march along z):
 //   f16-flow32 80^3 10.6 (20.4), 48^3 3.4 (14.4), 40^3 3.3 (10.3), 20^3 2.8 (8.2);
-//   f32 48^3 3.4 (12.3), 20^3 2.8 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
+//   f32 80^3 14.6 (20.5), 48^3 3.4 (12.3), 20^3 2.8 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
 // Small boxes are bound by the two exchanges (about 2.5 us: publish, poll, barriers). 80^3 is
 // bound by the latency of 12 warps of 168 registers (about 8,000 cycles of dual, 5,800 of primal)
-// and by the words' L2 traffic (3.6 MB per exchange each way).
+// and by the words' L2 traffic (3.6 MB per exchange each way). Its f32 form keeps p alone (90
+// registers of 168, 400 bytes spilled) and reads D (12 MB) and rho_c, gw (8 MB) from L2 in every
+// iteration; reading D one pair ahead took 15.5 us (12 more registers), 8 pairs by 256 threads 21.5.
 //
 // Boundaries (MIRROR with power-of-two 0.5/h only, see resident_ok in svs_solver.cu): central
 // differences vanish on a face and the adjoint sees q = 0 there, so with u mirrored into the cell
@@ -73,12 +75,13 @@ struct ResidentArgs {
 
 // Compiled shapes: NP voxel pairs per thread, up to NT threads; CU floats per component of u (with
 // its halo planes, rows and columns) and CQ of each of q_x (halo columns), q_y (halo rows) and
-// q_z (halo planes); up to NE face voxels per thread. KEEP_R: rho_c and the warped gradient stay
-// in registers (else they are read again in every iteration, before the wait for q's halo).
-template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_R_>
+// q_z (halo planes); up to NE face voxels per thread. KEEP_D, KEEP_R: the tensor, and rho_c and
+// the warped gradient, stay in registers; else they are read again in every iteration, D one pair
+// ahead of its use, the others before the wait for q's halo.
+template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_D_, bool KEEP_R_>
 struct ResShape {
   static constexpr int NP = NP_, NT = NT_, CU = CU_, CQ = CQ_, NE = NE_;
-  static constexpr bool KEEP_R = KEEP_R_;
+  static constexpr bool KEEP_D = KEEP_D_, KEEP_R = KEEP_R_;
   // the register file holds 16,384 registers per scheduler, a quarter of the warps each
   static constexpr int WARPS = (NT + 31) / 32, MAXREG = 16384 / ((WARPS + 3) / 4 * 32) / 8 * 8;
   static constexpr int REGS = MAXREG > 255 ? 255 : MAXREG;
@@ -248,7 +251,13 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
   const int dUQ = UXLO - QXLO;
   int o0 = (z0 + zl0) * gplane + (y0 + yl) * d.pitch + x0 + xl;
 
-  HT P[NP][9], D[NP][6], R[NP][4];
+  HT P[NP][9], D[C::KEEP_D ? NP : 1][6], R[NP][4];  // D not kept: one pair's
+  auto load_D = [&](int j) {
+    const int o = o0 + j * gplane;
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+      D[C::KEEP_D ? j : 0][c] = __ldg(reinterpret_cast<const HT*>(reinterpret_cast<const SP*>(d.D) + (long long)c * cs + o));
+  };
   auto load_R = [&](int j) {
     const int o = o0 + j * gplane;
     R[j][0] = __ldg(reinterpret_cast<const HT*>(reinterpret_cast<const SP*>(d.rc) + o));
@@ -262,7 +271,7 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
 #pragma unroll
     for (int c = 0; c < 9; ++c) P[j][c] = H::put(zero);
 #pragma unroll
-    for (int c = 0; c < 6; ++c) D[j][c] = H::put(zero);
+    for (int c = 0; c < 6; ++c) D[C::KEEP_D ? j : 0][c] = H::put(zero);
 #pragma unroll
     for (int c = 0; c < 4; ++c) R[j][c] = H::put(zero);
     if (j < nj) {
@@ -275,8 +284,7 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       };
 #pragma unroll
       for (int c = 0; c < 9; ++c) P[j][c] = take(d.p[a.src], c);
-#pragma unroll
-      for (int c = 0; c < 6; ++c) D[j][c] = take(d.D, c);
+      if constexpr (C::KEEP_D) load_D(j);
       if constexpr (C::KEEP_R) load_R(j);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -368,10 +376,12 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
   for (int it = 0; it < a.iters; ++it) {
     // keeps what is derived from these from being computed once, before the loop, and held
     asm volatile("" : "+r"(iu), "+r"(iqx), "+r"(aL), "+r"(aR), "+r"(dL), "+r"(dR), "+r"(o0), "+r"(nj));
+    if constexpr (C::KEEP_D) {
 #pragma unroll
-    for (int j = 0; j < NP; ++j)
+      for (int j = 0; j < NP; ++j)
 #pragma unroll
-      for (int c = 0; c < 6; ++c) H::pin(D[j][c]);
+        for (int c = 0; c < 6; ++c) H::pin(D[j][c]);
+    }
     const float sigma = next_sigma, tau = next_tau;
     if (it + 1 < a.iters) {
       next_sigma = __ldg(a.sig + it + 1);
@@ -385,6 +395,7 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       for (int j = 0; j < NP; ++j) {
         if (j < nj) {
           const int i = iu + j * PU;
+          if constexpr (!C::KEEP_D) load_D(j);
           // every read of u before the first write of q (the compiler cannot tell them apart)
           float2 e[3][3];
 #pragma unroll
@@ -397,7 +408,7 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
           }
           float2 Dk[6];
 #pragma unroll
-          for (int c = 0; c < 6; ++c) Dk[c] = H::get(D[j][c]);
+          for (int c = 0; c < 6; ++c) Dk[c] = H::get(D[C::KEEP_D ? j : 0][c]);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             float2 p0 = H::get(P[j][3 * c]), p1 = H::get(P[j][3 * c + 1]), p2 = H::get(P[j][3 * c + 2]);
@@ -504,16 +515,18 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
 }
 
 // Compiled shapes, every storage mode (svs_resident.cu).
-using ResSmall = ResShape<1, 512, 1920, 1408, 4, true>;
-using ResMid = ResShape<2, 512, 3456, 2688, 4, false>;
-using ResLarge = ResShape<5, 384, 5408, 4480, 4, false>;
+using ResSmall = ResShape<1, 512, 1920, 1408, 4, true, true>;
+using ResMid = ResShape<2, 512, 3456, 2688, 4, true, false>;
+// (5 pairs by 384 threads: 6 by 320 took 13.4 us at 80^3 f16-flow32, 8 by 256 11.9-14, against 10.6;
+// the register file is split by scheduler, so 13 to 16 warps would have 128 registers each)
+template <typename SP> using ResLarge = ResShape<5, 384, 5408, 4480, 4, sizeof(SP) == 2, false>;
 constexpr int kResShapes = 3, kResMaxWords = 2048;
 // Host view of a shape: voxel pairs and threads, floats per component, face words per thread.
 struct ResCaps {
   int np, nt, cu, cq, ne;
 };
 template <typename C> constexpr ResCaps res_caps() { return {C::NP, C::NT, C::CU, C::CQ, C::NE}; }
-constexpr ResCaps kResCaps[kResShapes] = {res_caps<ResSmall>(), res_caps<ResMid>(), res_caps<ResLarge>()};
+constexpr ResCaps kResCaps[kResShapes] = {res_caps<ResSmall>(), res_caps<ResMid>(), res_caps<ResLarge<__half>>()};
 
 // op 0: set the kernel's shared-memory attribute and return the CTAs one SM holds in *occ (false:
 // not usable); op 1: one cooperative launch of `grid` CTAs of `threads` threads on stream s.

@@ -1014,9 +1014,10 @@ double stream_us(int storage, double voxels) {
 // A resident launch with boxes of `threads` threads of `np` voxel pairs and `words` face words:
 // the two exchanges (2.5 us with next to no work), the warps' pairs, the words' traffic. 6x6x6
 // boxes 2.7 us, 8x8x10 3.4, 10x10x10 4.1 (np 1), 20x8x8 4.6, 20x10x10 6.1 (np 2; f32 5.3 and 6.9),
-// 16x12x20 10.6 (np 5).
+// 16x12x20 10.6 (np 5; f32 14.6).
 float resident_us(int storage, int np, int threads, int words) {
-  const float pair_us = np > 2 ? 0.12f : np == 2 && storage == SVS_STORAGE_F32 ? 0.11f : 0.085f;
+  const bool f32 = storage == SVS_STORAGE_F32;
+  const float pair_us = np > 2 ? (f32 ? 0.19f : 0.12f) : np == 2 && f32 ? 0.11f : 0.085f;
   return 2.45f + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words;
 }
 
