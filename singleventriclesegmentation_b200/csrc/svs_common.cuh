@@ -33,10 +33,11 @@ inline unsigned ceil_div(int64_t a, int64_t b) { return (unsigned)((a + b - 1) /
 // one volume length outside (boundary.cuh:33-46). The fold is a switch, not the reference's
 // device function-pointer table (boundary.cuh:54), so it inlines.
 __device__ __forceinline__ int fold(int i, int n, int bdry) {
-  int f;
-  if (bdry == SVS_BOUNDARY_MIRROR) f = i < 0 ? -i - 1 : (i > n - 1 ? 2 * n - 1 - i : i);
-  else if (bdry == SVS_BOUNDARY_NEAREST) f = i < 0 ? 0 : (i > n - 1 ? n - 1 : i);
-  else f = i < 0 ? -i : (i > n - 1 ? 2 * n - 2 - i : i);
+  int f = i;
+  if (bdry != SVS_BOUNDARY_NEAREST) {  // MIRROR repeats the face's node, REFLECT does not
+    const int s = bdry == SVS_BOUNDARY_MIRROR ? 1 : 0;
+    f = i > n - 1 ? 2 * n - 2 + s - i : max(i, -i - s);
+  }
   return min(max(f, 0), n - 1);
 }
 
@@ -85,7 +86,7 @@ using FieldRef = FieldRefT<float>;
 // Grid coordinate -> (floor index, fraction), the reference's floorf(c/h) and c/h - floor.
 template <typename T>
 __device__ __forceinline__ void split_coord(T c, T h, int& i, T& w) {
-  const T g = c / h;
+  const T g = h == T(1) ? c : c / h;
   i = (int)tfloor(g);
   w = g - (T)i;
 }
@@ -115,6 +116,103 @@ __device__ __forceinline__ T sample_cubic(const FieldRefT<T>& f, T cz, T cy, T c
     bz[dz] = hermite4(by[0], by[1], by[2], by[3], wy);
   }
   return hermite4(bz[0], bz[1], bz[2], bz[3], wz);
+}
+
+// hermite4 inside its window (w + 1 below 2) with t = (w + 1) - 1 given. The roundings are hermite4's
+// as compiled: halves and doubles are exact, so (b2 - b0) / 2, 2 pf - 2 pc and their sums are kept as
+// differences and scaled where they are used; -3 pf + 3 pc is one product and one fused multiply-add.
+template <typename T> __device__ __forceinline__ T hermite_one(T b0, T b1, T b2, T b3, T t) {
+  const T e0 = b2 - b0, e1 = b3 - b1;
+  const T a2 = fma(T(4), b1 - b2, e0) + e1;
+  const T b = fma(T(-0.5), e1, fma(T(3), b2, T(-3) * b1) - e0);
+  return fma(t, fma(t, fma(T(0.5) * t, a2, b), T(0.5) * e0), b1);
+}
+
+
+// ...and on two rows of samples at once: the packed FP32 instructions for float, one after the other
+// for double. Every operation rounds as its scalar counterpart.
+template <typename T> struct Two { T a, b; };
+__device__ __forceinline__ Two<float> two_add(Two<float> x, Two<float> y) {
+  const float2 r = __fadd2_rn(make_float2(x.a, x.b), make_float2(y.a, y.b));
+  return {r.x, r.y};
+}
+__device__ __forceinline__ Two<float> two_mul(float s, Two<float> x) {
+  const float2 r = __fmul2_rn(make_float2(s, s), make_float2(x.a, x.b));
+  return {r.x, r.y};
+}
+__device__ __forceinline__ Two<float> two_fma(float s, Two<float> x, Two<float> y) {
+  const float2 r = __ffma2_rn(make_float2(s, s), make_float2(x.a, x.b), make_float2(y.a, y.b));
+  return {r.x, r.y};
+}
+__device__ __forceinline__ Two<double> two_add(Two<double> x, Two<double> y) { return {x.a + y.a, x.b + y.b}; }
+__device__ __forceinline__ Two<double> two_mul(double s, Two<double> x) { return {s * x.a, s * x.b}; }
+__device__ __forceinline__ Two<double> two_fma(double s, Two<double> x, Two<double> y) {
+  return {fma(s, x.a, y.a), fma(s, x.b, y.b)};
+}
+template <typename T> __device__ __forceinline__ Two<T> two_sub(Two<T> x, Two<T> y) { return two_add(x, Two<T>{-y.a, -y.b}); }
+template <typename T>
+__device__ __forceinline__ Two<T> hermite_two(Two<T> b0, Two<T> b1, Two<T> b2, Two<T> b3, T t) {
+  const Two<T> e0 = two_sub(b2, b0), e1 = two_sub(b3, b1);
+  const Two<T> a2 = two_add(two_fma(T(4), two_sub(b1, b2), e0), e1);
+  const Two<T> b = two_fma(T(-0.5), e1, two_sub(two_fma(T(3), b2, two_mul(T(-3), b1)), e0));
+  return two_fma(t, two_fma(t, two_fma(T(0.5) * t, a2, b), two_mul(T(0.5), e0)), b1);
+}
+
+// Where one tricubic sample lies, found once for all fields sampled there: its window's first tap
+// and the position in the window per axis. `plain` is false where w + 1 rounds up to 2 on some axis:
+// hermite4's shifted window, left to sample_cubic.
+template <typename T>
+struct CubicTaps {
+  int x, y, z;
+  T tx, ty, tz;
+  bool plain;
+};
+template <typename T>
+__device__ __forceinline__ CubicTaps<T> cubic_taps(T cz, T cy, T cx, T hz, T hy, T hx) {
+  CubicTaps<T> k;
+  T wx, wy, wz;
+  split_coord(cx, hx, k.x, wx);
+  split_coord(cy, hy, k.y, wy);
+  split_coord(cz, hz, k.z, wz);
+  const T lx = wx + T(1), ly = wy + T(1), lz = wz + T(1);
+  --k.x, --k.y, --k.z;
+  k.tx = lx - T(1);
+  k.ty = ly - T(1);
+  k.tz = lz - T(1);
+  k.plain = lx < T(2) && ly < T(2) && lz < T(2);
+  return k;
+}
+// The sample of one field of fewer than 2^31 elements (x step sx). The four planes one after the
+// other (not unrolled): with all 64 loads in flight at once the sample takes 174 registers, and too
+// few warps are left to hide them (80^3: 40 us against 23).
+template <typename T>
+__device__ __forceinline__ T sample_cubic_taps(const T* __restrict__ f, const CubicTaps<T>& k, int nz, int ny, int nx, int sx,
+                                               int bdry) {
+  int xo[4], yo[4];
+#pragma unroll
+  for (int d = 0; d < 4; ++d) {
+    xo[d] = fold(k.x + d, nx, bdry) * sx;
+    yo[d] = fold(k.y + d, ny, bdry) * nx * sx;
+  }
+  T z0 = T(0), z1 = T(0), z2 = T(0), z3 = T(0);
+#pragma unroll 1
+  for (int dz = 0; dz < 4; ++dz) {
+    const T* p = f + fold(k.z + dz, nz, bdry) * (ny * nx * sx);
+    T by[4];
+#pragma unroll
+    for (int dy = 0; dy < 4; dy += 2) {
+      const T *r = p + yo[dy], *q = p + yo[dy + 1];
+      const Two<T> v = hermite_two(Two<T>{__ldg(r + xo[0]), __ldg(q + xo[0])}, Two<T>{__ldg(r + xo[1]), __ldg(q + xo[1])},
+                                   Two<T>{__ldg(r + xo[2]), __ldg(q + xo[2])}, Two<T>{__ldg(r + xo[3]), __ldg(q + xo[3])}, k.tx);
+      by[dy] = v.a;
+      by[dy + 1] = v.b;
+    }
+    z0 = z1;
+    z1 = z2;
+    z2 = z3;
+    z3 = hermite_one(by[0], by[1], by[2], by[3], k.ty);
+  }
+  return hermite_one(z0, z1, z2, z3, k.tz);
 }
 
 // Trilinear sample, interpolation_linear.cuh:250-295 (the 8 terms in the reference's order).

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <climits>
 #include <cstdio>
 #include <string>
 #include <vector>
@@ -229,6 +230,56 @@ __global__ void warp_cnn_kernel(const T* __restrict__ m, int B, int C, int nz, i
       out[((size_t)b * C + c) * nv + v] = sample(f, cz, cy, cx, hz, hy, hx, interp, bdry);
     }
   }
+}
+
+// Both warps for volumes whose launch fits a 3D grid (voxels of a plane, z, batch): 32-bit index
+// arithmetic, the sample's place found once for all channels. Channel c of voxel v of volume b is at
+// b*bs + c*cs + v*SX (SX = 0: sx, the field's interleaving). Bound by the instructions of a sample (21
+// cubics in the reference's coefficient form, kept operation for operation; folds and addresses) and
+// its 64 gathered loads through L1. Cubic, one channel: 80^3 40 -> 23 us, 8 x 96^3 516 -> 252 us;
+// linear 19 -> 11 and 219 -> 104 us. 8 x 4 voxels per warp with an unfolded form for warps inside the
+// volume: 21 and 287 us (twice the L1 lines per load).
+template <typename T, bool CUBIC, int SX>
+__global__ void __launch_bounds__(256, 4)
+warp_grid_kernel(const T* __restrict__ m, int C, int64_t bs, int64_t cs, int sx_arg, int nz, int ny, int nx,
+                 const T* __restrict__ phi, T hz, T hy, T hx, int interp, int bdry, T* __restrict__ out) {
+  const int sx = SX ? SX : sx_arg;
+  const int q = blockIdx.x * 256 + threadIdx.x;
+  const bool on = q < nx * ny;
+  const int y = q / nx, x = q - y * nx, z = blockIdx.y;
+  const int64_t nv = (int64_t)nz * ny * nx, v = ((int64_t)z * ny + (on ? y : 0)) * nx + (on ? x : 0);
+  const T* ph = phi + (blockIdx.z * nv + v) * 3;
+  const T cx = (T)x * hx + ph[0];
+  const T cy = (T)y * hy + ph[1];
+  const T cz = (T)z * hz + ph[2];
+  const T* src = m + blockIdx.z * bs;
+  T* dst = out + blockIdx.z * bs + v * sx;
+  if constexpr (CUBIC) {
+    const CubicTaps<T> k = cubic_taps(cz, cy, cx, hz, hy, hx);
+    if (on && k.plain) {
+      for (int c = 0; c < C; ++c) dst[c * cs] = sample_cubic_taps(src + c * cs, k, nz, ny, nx, sx, bdry);
+    } else if (on) {
+      for (int c = 0; c < C; ++c)
+        dst[c * cs] = sample_cubic(FieldRefT<T>{src + c * cs, nz, ny, nx, sx}, cz, cy, cx, hz, hy, hx, bdry);
+    }
+  } else if (on) {
+    for (int c = 0; c < C; ++c) {
+      const FieldRefT<T> f{src + c * cs, nz, ny, nx, sx};
+      dst[c * cs] = interp == SVS_INTERPOLATE_LINEAR ? sample_linear(f, cz, cy, cx, hz, hy, hx, bdry)
+                                                     : sample_nearest(f, cz, cy, cx, hz, hy, hx, bdry);
+    }
+  }
+}
+template <typename T>
+bool warp_grid(const T* m, int B, int C, int64_t bs, int64_t cs, int sx, int nz, int ny, int nx, const T* phi, T hz, T hy,
+               T hx, int interp, int bdry, T* out, cudaStream_t s) {
+  if (nz > 65535 || B > 65535 || (int64_t)nz * ny * nx * sx >= INT_MAX) return false;
+  const dim3 g(((unsigned)(nx * ny) + 255) / 256, (unsigned)nz, (unsigned)B);
+  const bool cubic = interp == SVS_INTERPOLATE_CUBIC_HERMITESPLINE;
+  auto k = cubic ? (sx == 1 ? warp_grid_kernel<T, true, 1> : sx == 3 ? warp_grid_kernel<T, true, 3> : warp_grid_kernel<T, true, 0>)
+                 : (sx == 1 ? warp_grid_kernel<T, false, 1> : warp_grid_kernel<T, false, 0>);
+  k<<<g, 256, 0, s>>>(m, C, bs, cs, sx, nz, ny, nx, phi, hz, hy, hx, interp, bdry, out);
+  return true;
 }
 
 // Prolongation3D: prolongationOps.cu:533-625. Target node i -> source coordinate (i*h_t)*L_s/L_t.
@@ -455,7 +506,8 @@ svs_status warp3d(const char* nm, const T* u, int nz, int ny, int nx, int C, con
   SVS_REQUIRE(valid_dims(nz, ny, nx) && C > 0, std::string(nm) + ": bad sizes");
   SVS_REQUIRE(valid_bdry(boundary) && valid_interp(interpolation), std::string(nm) + ": bad mode");
   const int64_t n = (int64_t)nz * ny * nx;
-  warp_kernel<T><<<grid_for(n), kThreads, 0, stream>>>(u, nz, ny, nx, C, phi, hz, hy, hx, interpolation, boundary, out);
+  if (!warp_grid<T>(u, 1, C, 0, 1, C, nz, ny, nx, phi, hz, hy, hx, interpolation, boundary, out, stream))
+    warp_kernel<T><<<grid_for(n), kThreads, 0, stream>>>(u, nz, ny, nx, C, phi, hz, hy, hx, interpolation, boundary, out);
   return check_launch(nm);
 }
 
@@ -480,9 +532,10 @@ svs_status warp_cnn3d(const char* nm, const T* m, int B, int C, int nz, int ny, 
   SVS_REQUIRE(m && phi && out, std::string(nm) + ": null pointer");
   SVS_REQUIRE(valid_dims(nz, ny, nx) && B > 0 && C > 0, std::string(nm) + ": bad sizes");
   SVS_REQUIRE(valid_bdry(boundary) && valid_interp(interpolation), std::string(nm) + ": bad mode");
-  const int64_t n = (int64_t)nz * ny * nx * B;
-  warp_cnn_kernel<T><<<grid_for(n), kThreads, 0, stream>>>(m, B, C, nz, ny, nx, phi, hz, hy, hx, interpolation,
-                                                            boundary, out);
+  const int64_t nv = (int64_t)nz * ny * nx, n = nv * B;
+  if (!warp_grid<T>(m, B, C, nv * C, nv, 1, nz, ny, nx, phi, hz, hy, hx, interpolation, boundary, out, stream))
+    warp_cnn_kernel<T><<<grid_for(n), kThreads, 0, stream>>>(m, B, C, nz, ny, nx, phi, hz, hy, hx, interpolation,
+                                                              boundary, out);
   return check_launch(nm);
 }
 
