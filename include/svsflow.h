@@ -127,6 +127,12 @@ svs_status svs_warp_cnn3d(const float* m, int B, int C, int nz, int ny, int nx, 
 svs_status svs_prolongate3d(const float* u, int nz, int ny, int nx, int C, float lz, float ly,
                             float lx, int tz, int ty, int tx, float tlz, float tly, float tlx,
                             int interpolation, int boundary, float* out, svs_stream_t stream);
+/* The same into C_out components per target voxel, those from C on zero (fewer: the first C_out):
+ * a resampled time axis padded in one pass (prolongation.py:15-22, 83). */
+svs_status svs_prolongate3d_padded(const float* u, int nz, int ny, int nx, int C, float lz, float ly,
+                                   float lx, int tz, int ty, int tx, float tlz, float tly, float tlx,
+                                   int interpolation, int boundary, int C_out, float* out,
+                                   svs_stream_t stream);
 
 /* apply_gaussian_blur3d (svs/utils/flow_utils.py:94-112): zero-padded 3D correlation of
  * in [NZ,NY,NX] with a (2r+1)^3 kernel given in HOST memory (weights_host, float32). */
@@ -166,6 +172,10 @@ svs_status svs_warp_cnn3d_f64(const double* m, int B, int C, int nz, int ny, int
 svs_status svs_prolongate3d_f64(const double* u, int nz, int ny, int nx, int C, double lz, double ly,
                                 double lx, int tz, int ty, int tx, double tlz, double tly, double tlx,
                                 int interpolation, int boundary, double* out, svs_stream_t stream);
+svs_status svs_prolongate3d_padded_f64(const double* u, int nz, int ny, int nx, int C, double lz, double ly,
+                                       double lx, int tz, int ty, int tx, double tlz, double tly, double tlx,
+                                       int interpolation, int boundary, int C_out, double* out,
+                                       svs_stream_t stream);
 svs_status svs_gauss_blur3d_f64(const double* in, int nz, int ny, int nx, const double* weights_host, int r,
                                 double* out, svs_stream_t stream);
 svs_status svs_median3d_f64(const double* in, int nz, int ny, int nx, int C, int ks, double* out,

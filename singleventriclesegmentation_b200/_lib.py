@@ -64,6 +64,7 @@ _SIGS = {
     "svs_warp3d_backward": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "svs_warp_cnn3d": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p]),
     "svs_prolongate3d": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p]),
+    "svs_prolongate3d_padded": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_void_p, c_void_p]),
     "svs_gauss_blur3d": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p]),
     "svs_median3d": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "svs_nabla3d_forward_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_double, c_double, c_double, c_int, c_void_p, c_void_p]),
@@ -76,6 +77,7 @@ _SIGS = {
     "svs_warp3d_backward_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_double, c_double, c_double, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "svs_warp_cnn3d_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_double, c_double, c_double, c_int, c_int, c_void_p, c_void_p]),
     "svs_prolongate3d_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_double, c_double, c_double, c_int, c_int, c_int, c_double, c_double, c_double, c_int, c_int, c_void_p, c_void_p]),
+    "svs_prolongate3d_padded_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_double, c_double, c_double, c_int, c_int, c_int, c_double, c_double, c_double, c_int, c_int, c_int, c_void_p, c_void_p]),
     "svs_gauss_blur3d_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p]),
     "svs_median3d_f64": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "svs_tvl1_plan_create": (c_int, [ctypes.POINTER(TVL1Params), c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_void_p)]),

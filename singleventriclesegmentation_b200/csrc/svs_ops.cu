@@ -287,7 +287,7 @@ template <typename T>
 __global__ void prolongate_kernel(const T* __restrict__ u, int nz, int ny, int nx, int C,
                                   T lz, T ly, T lx, T hz, T hy, T hx,
                                   int tz, int ty, int tx, T tlz, T tly, T tlx,
-                                  T thz, T thy, T thx, int interp, int bdry,
+                                  T thz, T thy, T thx, int interp, int bdry, int CO,
                                   T* __restrict__ out) {
   const int64_t n = (int64_t)tz * ty * tx;
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n;
@@ -296,13 +296,110 @@ __global__ void prolongate_kernel(const T* __restrict__ u, int nz, int ny, int n
     const T cx = (T)x * thx * lx / tlx;
     const T cy = (T)y * thy * ly / tly;
     const T cz = (T)z * thz * lz / tlz;
-    for (int c = 0; c < C; ++c) {
+    for (int c = 0; c < min(C, CO); ++c) {
       FieldRefT<T> f{u + c, nz, ny, nx, C};
-      out[v * C + c] = sample(f, cz, cy, cx, hz, hy, hx, interp, bdry);
+      out[v * CO + c] = sample(f, cz, cy, cx, hz, hy, hx, interp, bdry);
     }
   }
 }
 
+
+// The same for targets whose launch fits a 2D grid (components and voxels of a plane, z), cubic and
+// nearest: one thread per output component, components fastest, so that a warp reads and writes
+// consecutive components (one thread per voxel strode over them). CO components are written per
+// voxel, those from C on zero (a time axis padded in the same pass). Cubic, 40^3 -> 80^3: 9 components
+// 226 -> 162 us, 3 86 -> 58 us.
+template <typename T, bool CUBIC>
+__global__ void __launch_bounds__(256)
+prolongate_grid_kernel(const T* __restrict__ u, int nz, int ny, int nx, int C, T lz, T ly, T lx, T hz, T hy, T hx, int ty,
+                       int tx, T tlz, T tly, T tlx, T thz, T thy, T thx, int bdry, int CO, T* __restrict__ out) {
+  const int e = blockIdx.x * 256 + threadIdx.x;
+  if (e >= ty * tx * CO) return;
+  const int q = e / CO, c = e - q * CO, y = q / tx, x = q - y * tx, z = blockIdx.y;
+  T v = T(0);
+  if (c < C) {
+    const T cx = (T)x * thx * lx / tlx;
+    const T cy = (T)y * thy * ly / tly;
+    const T cz = (T)z * thz * lz / tlz;
+    const FieldRefT<T> f{u + c, nz, ny, nx, C};
+    if constexpr (CUBIC) {
+      const CubicTaps<T> k = cubic_taps(cz, cy, cx, hz, hy, hx);
+      v = k.plain ? sample_cubic_taps(u + c, k, nz, ny, nx, C, bdry) : sample_cubic(f, cz, cy, cx, hz, hy, hx, bdry);
+    } else {
+      v = sample_nearest(f, cz, cy, cx, hz, hy, hx, bdry);
+    }
+  }
+  out[(int64_t)z * ty * tx * CO + e] = v;
+}
+
+__device__ __forceinline__ float trn_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double trn_mul(double a, double b) { return __dmul_rn(a, b); }
+
+// Trilinear: a thread owns one output component of one (y, x) and walks kZRun target planes, so that
+// its taps along x and y, with their divisions, are found once, and a source plane's four values are
+// read once for all the targets between two planes (a cine's few slices become many). The sums are
+// sample_linear's, term by term. 16x160x160x25 -> 80^3 x 25 341 us (one thread per voxel, strided),
+// 168 (one per output), 117 (one block per row: 410 MB through L2) -> 37 us; padded to 35 components 56.
+constexpr int kZRun = 16;
+template <typename T>
+__global__ void __launch_bounds__(256)
+prolongate_linear_kernel(const T* __restrict__ u, int nz, int ny, int nx, int C, T lz, T ly, T lx, T hz, T hy, T hx, int tz,
+                         int ty, int tx, T tlz, T tly, T tlx, T thz, T thy, T thx, int bdry, int CO, T* __restrict__ out) {
+  __shared__ int s0[kZRun], s1[kZRun];
+  __shared__ T sw[kZRun];
+  const int zb = blockIdx.y * kZRun, ze = min(zb + kZRun, tz);
+  if (threadIdx.x < ze - zb) {
+    int i;
+    T w;
+    split_coord((T)(zb + threadIdx.x) * thz * lz / tlz, hz, i, w);
+    s0[threadIdx.x] = fold(i, nz, bdry);
+    s1[threadIdx.x] = fold(i + 1, nz, bdry);
+    sw[threadIdx.x] = w;
+  }
+  __syncthreads();
+  const int e = blockIdx.x * 256 + threadIdx.x;
+  if (e >= ty * tx * CO) return;
+  const int q = e / CO, c = e - q * CO, y = q / tx, x = q - y * tx;
+  T* dst = out + (int64_t)zb * ty * tx * CO + e;
+  const int64_t step = (int64_t)ty * tx * CO;
+  if (c >= C) {
+    for (int z = zb; z < ze; ++z, dst += step) *dst = T(0);
+    return;
+  }
+  int ix, iy;
+  T wx, wy;
+  split_coord((T)x * thx * lx / tlx, hx, ix, wx);
+  split_coord((T)y * thy * ly / tly, hy, iy, wy);
+  const int64_t y0 = (int64_t)fold(iy, ny, bdry) * nx, y1 = (int64_t)fold(iy + 1, ny, bdry) * nx;
+  const int x0 = fold(ix, nx, bdry), x1 = fold(ix + 1, nx, bdry);
+  const int64_t o[4] = {(y0 + x0) * C + c, (y0 + x1) * C + c, (y1 + x0) * C + c, (y1 + x1) * C + c};
+  const int64_t plane = (int64_t)ny * nx * C;
+  T f0[4], f1[4];  // the values at y0x0, y0x1, y1x0, y1x1 of the two source planes
+  int p0 = -1, p1 = -1;
+  for (int z = zb; z < ze; ++z, dst += step) {
+    const int z0 = s0[z - zb], z1 = s1[z - zb];
+    if (z0 != p0) {
+      const bool shift = z0 == p1;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) f0[k] = shift ? f1[k] : __ldg(u + z0 * plane + o[k]);
+      p0 = z0;
+    }
+    if (z1 != p1) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) f1[k] = __ldg(u + z1 * plane + o[k]);
+      p1 = z1;
+    }
+    const T wz = sw[z - zb];
+    T v = fma((1 - wz) * (1 - wy) * (1 - wx), f0[0], trn_mul(wz * (1 - wy) * (1 - wx), f1[0]));
+    v = fma((1 - wz) * (1 - wy) * wx, f0[1], v);
+    v = fma(wz * (1 - wy) * wx, f1[1], v);
+    v = fma((1 - wz) * wy * (1 - wx), f0[2], v);
+    v = fma(wz * wy * (1 - wx), f1[2], v);
+    v = fma((1 - wz) * wy * wx, f0[3], v);
+    v = fma(wz * wy * wx, f1[3], v);
+    *dst = v;
+  }
+}
 
 // ------------------------------------------------------------------------------ warp backward
 // Catmull-Rom basis weights at fraction w (the d_out_d_p_* of
@@ -541,9 +638,9 @@ svs_status warp_cnn3d(const char* nm, const T* m, int B, int C, int nz, int ny, 
 
 template <typename T>
 svs_status prolongate3d(const char* nm, const T* u, int nz, int ny, int nx, int C, T lz, T ly, T lx, int tz, int ty,
-                        int tx, T tlz, T tly, T tlx, int interpolation, int boundary, T* out, cudaStream_t stream) {
+                        int tx, T tlz, T tly, T tlx, int interpolation, int boundary, int CO, T* out, cudaStream_t stream) {
   SVS_REQUIRE(u && out, std::string(nm) + ": null pointer");
-  SVS_REQUIRE(valid_dims(nz, ny, nx) && valid_dims(tz, ty, tx) && C > 0, std::string(nm) + ": bad sizes");
+  SVS_REQUIRE(valid_dims(nz, ny, nx) && valid_dims(tz, ty, tx) && C > 0 && CO > 0, std::string(nm) + ": bad sizes");
   SVS_REQUIRE(nz > 1 && ny > 1 && nx > 1 && tz > 1 && ty > 1 && tx > 1,
               std::string(nm) + ": meshes need at least 2 nodes per axis (h = L/(N-1))");
   SVS_REQUIRE(valid_bdry(boundary) && valid_interp(interpolation), std::string(nm) + ": bad mode");
@@ -551,8 +648,24 @@ svs_status prolongate3d(const char* nm, const T* u, int nz, int ny, int nx, int 
   const T hz = lz / (T)(nz - 1), hy = ly / (T)(ny - 1), hx = lx / (T)(nx - 1);
   const T thz = tlz / (T)(tz - 1), thy = tly / (T)(ty - 1), thx = tlx / (T)(tx - 1);
   const int64_t n = (int64_t)tz * ty * tx;
+  if (tz <= 65535 && (int64_t)ty * tx * CO < INT_MAX - 256 && (int64_t)nz * ny * nx * C < INT_MAX) {
+    if (interpolation == SVS_INTERPOLATE_LINEAR) {
+      const dim3 g((unsigned)((int64_t)ty * tx * CO + 255) / 256, (unsigned)(tz + kZRun - 1) / kZRun);
+      prolongate_linear_kernel<T><<<g, 256, 0, stream>>>(u, nz, ny, nx, C, lz, ly, lx, hz, hy, hx, tz, ty, tx, tlz, tly, tlx,
+                                                         thz, thy, thx, boundary, CO, out);
+      return check_launch(nm);
+    }
+    const dim3 g((unsigned)((int64_t)ty * tx * CO + 255) / 256, (unsigned)tz);
+    auto k = interpolation == SVS_INTERPOLATE_CUBIC_HERMITESPLINE ? prolongate_grid_kernel<T, true> : prolongate_grid_kernel<T, false>;
+    k<<<g, 256, 0, stream>>>(u, nz, ny, nx, C, lz, ly, lx, hz, hy, hx, ty, tx, tlz, tly, tlx, thz, thy, thx, boundary, CO, out);
+    return check_launch(nm);
+  }
+  if (CO > C) {
+    svs_status st = check_cuda(cudaMemsetAsync(out, 0, n * CO * sizeof(T), stream), nm);
+    if (st) return st;
+  }
   prolongate_kernel<T><<<grid_for(n), kThreads, 0, stream>>>(u, nz, ny, nx, C, lz, ly, lx, hz, hy, hx, tz, ty, tx, tlz,
-                                                              tly, tlx, thz, thy, thx, interpolation, boundary, out);
+                                                              tly, tlx, thz, thy, thx, interpolation, boundary, CO, out);
   return check_launch(nm);
 }
 
@@ -638,11 +751,19 @@ svs_status svs_warp_cnn3d_f64(const double* m, int B, int C, int nz, int ny, int
 }
 
 svs_status svs_prolongate3d(const float* u, int nz, int ny, int nx, int C, float lz, float ly, float lx, int tz, int ty, int tx, float tlz, float tly, float tlx, int interpolation, int boundary, float* out, svs_stream_t stream) {
-  return prolongate3d<float>("svs_prolongate3d", u, nz, ny, nx, C, lz, ly, lx, tz, ty, tx, tlz, tly, tlx, interpolation, boundary, out, stream);
+  return prolongate3d<float>("svs_prolongate3d", u, nz, ny, nx, C, lz, ly, lx, tz, ty, tx, tlz, tly, tlx, interpolation, boundary, C, out, stream);
+}
+
+svs_status svs_prolongate3d_padded(const float* u, int nz, int ny, int nx, int C, float lz, float ly, float lx, int tz, int ty, int tx, float tlz, float tly, float tlx, int interpolation, int boundary, int C_out, float* out, svs_stream_t stream) {
+  return prolongate3d<float>("svs_prolongate3d_padded", u, nz, ny, nx, C, lz, ly, lx, tz, ty, tx, tlz, tly, tlx, interpolation, boundary, C_out, out, stream);
 }
 
 svs_status svs_prolongate3d_f64(const double* u, int nz, int ny, int nx, int C, double lz, double ly, double lx, int tz, int ty, int tx, double tlz, double tly, double tlx, int interpolation, int boundary, double* out, svs_stream_t stream) {
-  return prolongate3d<double>("svs_prolongate3d_f64", u, nz, ny, nx, C, lz, ly, lx, tz, ty, tx, tlz, tly, tlx, interpolation, boundary, out, stream);
+  return prolongate3d<double>("svs_prolongate3d_f64", u, nz, ny, nx, C, lz, ly, lx, tz, ty, tx, tlz, tly, tlx, interpolation, boundary, C, out, stream);
+}
+
+svs_status svs_prolongate3d_padded_f64(const double* u, int nz, int ny, int nx, int C, double lz, double ly, double lx, int tz, int ty, int tx, double tlz, double tly, double tlx, int interpolation, int boundary, int C_out, double* out, svs_stream_t stream) {
+  return prolongate3d<double>("svs_prolongate3d_padded_f64", u, nz, ny, nx, C, lz, ly, lx, tz, ty, tx, tlz, tly, tlx, interpolation, boundary, C_out, out, stream);
 }
 
 }  // extern "C"

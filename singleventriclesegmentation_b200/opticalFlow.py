@@ -288,17 +288,18 @@ class Prolongation3D:
         self._interp = int(interpolation)
         self._bdry = int(boundary)
 
-    def _run(self, u, tail):
+    def _run(self, u, tail, out_components=None):
         nz, ny, nx = u.shape[:3]
         C = int(np.prod(tail)) if tail else 1
         d = self._dst
         tz, ty, tx = d.getNZ(), d.getNY(), d.getNX()
-        out = torch.empty((tz, ty, tx) + tuple(tail), dtype=u.dtype, device=u.device)
+        co = C if out_components is None else int(out_components)
+        out = torch.empty((tz, ty, tx) + (tuple(tail) if out_components is None else (co,)), dtype=u.dtype, device=u.device)
         s = self._src
         with torch.cuda.device(u.device):
-            check(_op("svs_prolongate3d", u)(ptr(u), nz, ny, nx, C, s.getLZ(), s.getLY(), s.getLX(),
-                                              tz, ty, tx, d.getLZ(), d.getLY(), d.getLX(), self._interp,
-                                              self._bdry, ptr(out), stream_ptr(u.device)))
+            check(_op("svs_prolongate3d_padded", u)(ptr(u), nz, ny, nx, C, s.getLZ(), s.getLY(), s.getLX(),
+                                                     tz, ty, tx, d.getLZ(), d.getLY(), d.getLX(), self._interp,
+                                                     self._bdry, co, ptr(out), stream_ptr(u.device)))
         return out
 
     def forward(self, u: torch.Tensor) -> torch.Tensor:
@@ -310,6 +311,13 @@ class Prolongation3D:
         _check_input(u, "u")
         _check_dim(u, 4)
         return self._run(u, (u.shape[3],))
+
+    def forwardVectorFieldPadded(self, u: torch.Tensor, components: int) -> torch.Tensor:
+        """forwardVectorField into `components` components, those beyond u's zero (fewer: the first
+        ones), in one pass."""
+        _check_input(u, "u")
+        _check_dim(u, 4)
+        return self._run(u, (u.shape[3],), components)
 
     def forwardMatrixField(self, u: torch.Tensor) -> torch.Tensor:
         _check_input(u, "u")

@@ -43,6 +43,7 @@ def resample_patient(img_zyxt: torch.Tensor, seg_dia_zyx: Optional[torch.Tensor]
     op = opticalFlow.Prolongation3D(old, new, interp, bdry)
     seg_dia = op.forward(seg_dia_zyx.float().contiguous()).round() if seg_dia_zyx is not None else None
     seg_sys = op.forward(seg_sys_zyx.float().contiguous()).round() if seg_sys_zyx is not None else None
-    img = time_pading(pad_time, op.forwardVectorField(img_zyxt.float().contiguous()))
+    img = img_zyxt.float().contiguous()
+    img = op.forwardVectorFieldPadded(img, pad_time) if pad_time > 0 else time_pading(pad_time, op.forwardVectorField(img))
     factors = (NX / nx, NY / ny, NZ / nz, pad_time / nt)
     return img, seg_dia, seg_sys, factors

@@ -1,5 +1,5 @@
-"""Edges of the grid kernels of the resampling operators: the warps where a block ends, against the
-oracle."""
+"""Edges of the grid kernels of the resampling operators: the warps and the prolongation where a block,
+a run of z planes or a component row ends, against the oracle; padded and cropped time axes."""
 import numpy as np
 import pytest
 import torch
@@ -34,3 +34,23 @@ def test_warp_edges(cuda, oracle, of, interp, shape):
     got = op.forward(T(m), T(phi)).cpu().numpy()
     want = oracle.warp_cnn(m, phi, h, interp, "MIRROR")
     np.testing.assert_allclose(got, want, rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("interp", ["NEAREST", "LINEAR", "CUBIC_HERMITESPLINE"])
+@pytest.mark.parametrize("src,dst,C", [((3, 9, 8), (17, 6, 11), 1), ((16, 5, 7), (16, 8, 9), 3), ((5, 6, 7), (33, 4, 3), 25),
+                                       ((20, 7, 6), (7, 5, 4), 9)])
+def test_prolongation_edges(cuda, oracle, of, interp, src, dst, C):
+    """z runs of exactly 16 and one more, planes shared by several targets and skipped between them,
+    component rows that end inside a block."""
+    rng = np.random.default_rng(C)
+    u = rng.standard_normal(src + (C,)).astype(np.float32)
+    old, new = of.MeshInfo3D(*src, *(s - 1 for s in src)), of.MeshInfo3D(*dst, *(s - 1 for s in dst))
+    op = of.Prolongation3D(old, new, getattr(of, "INTERPOLATE_" + interp), of.BOUNDARY_MIRROR)
+    got = op.forwardVectorField(T(u))
+    one = of.Prolongation3D(old, new, getattr(of, "INTERPOLATE_" + interp), of.BOUNDARY_MIRROR)
+    for c in range(C):
+        assert torch.equal(one.forward(T(u[..., c])), got[..., c])
+    want = oracle.prolongate(u, tuple(float(s - 1) for s in src), dst, tuple(float(s - 1) for s in dst), interp, "MIRROR")
+    np.testing.assert_allclose(got.cpu().numpy(), want, rtol=2e-5, atol=2e-5)
+    for n in (1, C, C + 6):
+        assert torch.equal(op.forwardVectorFieldPadded(T(u), n), torch.nn.functional.pad(got, (0, n - C)))
