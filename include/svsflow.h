@@ -121,6 +121,16 @@ svs_status svs_warp_cnn3d(const float* m, int B, int C, int nz, int ny, int nx, 
                           float hz, float hy, float hx, int interpolation, int boundary,
                           float* out, svs_stream_t stream);
 
+/* warping.py:205-243 (_propagate): the first mask carried through `steps` forward flows and the last
+ * through the backward ones ([steps,NZ,NY,NX,3] each, WarpingCNN3D.forward per step on the float
+ * volumes), both chains thresholded at 0.5 into [steps+1,NZ,NY,NX], the backward chain reversed.
+ * scratch: 4 NZ NY NX floats of device memory (unused for steps = 0). */
+svs_status svs_propagate_masks3d(const float* first, const float* last, const float* forward_flow,
+                                 const float* backward_flow, int steps, int nz, int ny, int nx,
+                                 float hz, float hy, float hx, int interpolation, int boundary,
+                                 float* scratch, float* forward_masks, float* backward_masks,
+                                 svs_stream_t stream);
+
 /* Prolongation3D.forward / .forwardVectorField / .forwardMatrixField (prolongationOps.h:79-107;
  * kernels prolongationOps.cu:533-625): resample a C-component field from mesh (n*, L*) to mesh
  * (t*, tL*); target node i samples the source at (i*h_t)*L_s/L_t. */

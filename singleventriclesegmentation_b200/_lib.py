@@ -63,6 +63,7 @@ _SIGS = {
     "svs_warp3d": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p]),
     "svs_warp3d_backward": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "svs_warp_cnn3d": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p]),
+    "svs_propagate_masks3d": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "svs_prolongate3d": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p]),
     "svs_prolongate3d_padded": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_void_p, c_void_p]),
     "svs_gauss_blur3d": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p]),
@@ -148,6 +149,26 @@ def check(status: int) -> None:
     if status != SVS_OK:
         msg = lib().svs_last_error()
         raise SVSError(status, msg.decode() if msg else "")
+
+
+_bound = {}
+
+
+def call(name: str, t: torch.Tensor, *args) -> None:
+    """Entry point `name` for t's value type (float32: name, float64: name_f64; the reference
+    dispatched both) with `args` and t's device's current stream, on that device."""
+    key = (name, t.dtype)
+    fn = _bound.get(key)
+    if fn is None:
+        fn = _bound[key] = getattr(lib(), name + ("_f64" if t.dtype == torch.float64 else ""))
+    dev = t.get_device()
+    if dev == torch._C._cuda_getDevice():
+        status = fn(*args, torch._C._cuda_getCurrentRawStream(dev))
+    else:
+        with torch.cuda.device(dev):
+            status = fn(*args, torch._C._cuda_getCurrentRawStream(dev))
+    if status != SVS_OK:
+        check(status)
 
 
 def stream_ptr(device=None) -> int:

@@ -270,6 +270,43 @@ warp_grid_kernel(const T* __restrict__ m, int C, int64_t bs, int64_t cs, int sx_
     }
   }
 }
+// One step of the two mask chains of a patient (blockIdx.z: forward, backward): each chain's volume
+// warped by its flow, kept as it is for the next step and written thresholded at 0.5 to its place in
+// the result. One launch a step instead of two warps, and no passes over the results afterwards.
+struct MaskStep {
+  const float *src[2], *phi[2];
+  float *dst[2], *mask[2];
+};
+template <bool CUBIC>
+__global__ void __launch_bounds__(256, 4)
+mask_step_kernel(const __grid_constant__ MaskStep k, int nz, int ny, int nx, float hz, float hy, float hx, int interp,
+                 int bdry) {
+  const int q = blockIdx.x * 256 + threadIdx.x;
+  if (q >= nx * ny) return;
+  const int y = q / nx, x = q - y * nx, z = blockIdx.y;
+  const int64_t v = (int64_t)z * ny * nx + q;
+  const float* ph = k.phi[blockIdx.z] + 3 * v;
+  const float* src = k.src[blockIdx.z];
+  const float cx = (float)x * hx + ph[0];
+  const float cy = (float)y * hy + ph[1];
+  const float cz = (float)z * hz + ph[2];
+  const FieldRef f{src, nz, ny, nx, 1};
+  float m;
+  if constexpr (CUBIC) {
+    const CubicTaps<float> t = cubic_taps(cz, cy, cx, hz, hy, hx);
+    m = t.plain ? sample_cubic_taps(src, t, nz, ny, nx, 1, bdry) : sample_cubic(f, cz, cy, cx, hz, hy, hx, bdry);
+  } else {
+    m = interp == SVS_INTERPOLATE_LINEAR ? sample_linear(f, cz, cy, cx, hz, hy, hx, bdry)
+                                         : sample_nearest(f, cz, cy, cx, hz, hy, hx, bdry);
+  }
+  k.dst[blockIdx.z][v] = m;
+  k.mask[blockIdx.z][v] = m > 0.5f ? 1.f : 0.f;
+}
+__global__ void mask_threshold_kernel(const __grid_constant__ MaskStep k, int64_t n) {
+  const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (v < n) k.mask[blockIdx.y][v] = k.src[blockIdx.y][v] > 0.5f ? 1.f : 0.f;
+}
+
 template <typename T>
 bool warp_grid(const T* m, int B, int C, int64_t bs, int64_t cs, int sx, int nz, int ny, int nx, const T* phi, T hz, T hy,
                T hx, int interp, int bdry, T* out, cudaStream_t s) {
@@ -740,6 +777,33 @@ svs_status svs_warp3d_backward(const float* u, int nz, int ny, int nx, const flo
 
 svs_status svs_warp3d_backward_f64(const double* u, int nz, int ny, int nx, const double* phi, const double* grad_out, double hz, double hy, double hx, int interpolation, int boundary, double* grad_u, double* grad_phi, svs_stream_t stream) {
   return warp3d_backward<double>("svs_warp3d_backward_f64", u, nz, ny, nx, phi, grad_out, hz, hy, hx, interpolation, boundary, grad_u, grad_phi, stream);
+}
+
+svs_status svs_propagate_masks3d(const float* first, const float* last, const float* forward_flow,
+                                 const float* backward_flow, int steps, int nz, int ny, int nx, float hz, float hy, float hx,
+                                 int interpolation, int boundary, float* scratch, float* forward_masks,
+                                 float* backward_masks, svs_stream_t stream) {
+  const char* nm = "svs_propagate_masks3d";
+  SVS_REQUIRE(first && last && forward_masks && backward_masks, std::string(nm) + ": null pointer");
+  SVS_REQUIRE(steps >= 0 && (steps == 0 || (forward_flow && backward_flow && scratch)), std::string(nm) + ": null pointer");
+  SVS_REQUIRE(valid_dims(nz, ny, nx), std::string(nm) + ": bad sizes");
+  SVS_REQUIRE(valid_bdry(boundary) && valid_interp(interpolation), std::string(nm) + ": bad mode");
+  const int64_t n = (int64_t)nz * ny * nx;
+  if (nz > 65535 || n >= INT_MAX) return fail(SVS_ERR_UNSUPPORTED, std::string(nm) + ": volume too large");
+  MaskStep k{{first, last}, {nullptr, nullptr}, {nullptr, nullptr}, {forward_masks, backward_masks + steps * n}};
+  mask_threshold_kernel<<<dim3(ceil_div(n, 256), 2), 256, 0, stream>>>(k, n);
+  const dim3 g((unsigned)(ny * nx + 255) / 256, (unsigned)nz, 2);
+  auto step = interpolation == SVS_INTERPOLATE_CUBIC_HERMITESPLINE ? mask_step_kernel<true> : mask_step_kernel<false>;
+  for (int t = 0; t < steps; ++t) {
+    for (int c = 0; c < 2; ++c) {
+      k.phi[c] = (c ? backward_flow : forward_flow) + 3 * n * t;
+      k.dst[c] = scratch + (2 * c + (t & 1)) * n;
+      k.mask[c] = c ? backward_masks + (steps - 1 - t) * n : forward_masks + (t + 1) * n;
+    }
+    step<<<g, 256, 0, stream>>>(k, nz, ny, nx, hz, hy, hx, interpolation, boundary);
+    for (int c = 0; c < 2; ++c) k.src[c] = k.dst[c];
+  }
+  return check_launch(nm, 1 + (uint64_t)steps);
 }
 
 svs_status svs_warp_cnn3d(const float* m, int B, int C, int nz, int ny, int nx, const float* phi, float hz, float hy, float hx, int interpolation, int boundary, float* out, svs_stream_t stream) {

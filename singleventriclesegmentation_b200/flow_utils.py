@@ -11,9 +11,8 @@ from typing import Tuple
 import numpy as np
 import torch
 
-from . import _lib
 from . import opticalFlow
-from ._lib import check, ptr, stream_ptr
+from ._lib import call, ptr
 
 
 def get_interpolation_type(inter_type_str: str, bound_type_str: str):
@@ -68,9 +67,7 @@ def apply_gaussian_blur3d(vol: torch.Tensor, sigma: float) -> torch.Tensor:
     r = w.shape[0] // 2
     out = torch.empty_like(vol)
     nz, ny, nx = vol.shape
-    fn = _lib.lib().svs_gauss_blur3d_f64 if f64 else _lib.lib().svs_gauss_blur3d
-    with torch.cuda.device(vol.device):
-        check(fn(ptr(vol), nz, ny, nx, w.ctypes.data, r, ptr(out), stream_ptr(vol.device)))
+    call("svs_gauss_blur3d", vol, ptr(vol), nz, ny, nx, w.ctypes.data, r, ptr(out))
     return out
 
 
@@ -84,9 +81,7 @@ def apply_median_filter(u: torch.Tensor, ks: int, device: torch.device = None) -
     nz, ny, nx = x.shape[:3]
     C = 1 if x.dim() == 3 else int(np.prod(x.shape[3:]))
     out = torch.empty_like(x)
-    fn = _lib.lib().svs_median3d_f64 if x.dtype == torch.float64 else _lib.lib().svs_median3d
-    with torch.cuda.device(x.device):
-        check(fn(ptr(x), nz, ny, nx, C, int(ks), ptr(out), stream_ptr(x.device)))
+    call("svs_median3d", x, ptr(x), nz, ny, nx, C, int(ks), ptr(out))
     return out if device is None else out.to(device)
 
 

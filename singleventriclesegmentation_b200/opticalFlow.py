@@ -12,12 +12,13 @@ Argument errors raise RuntimeError, as the reference's TORCH_CHECK / CHECK_INPUT
 from __future__ import annotations
 
 import enum
+import math
 
 import numpy as np
 import torch
 
 from . import _lib
-from ._lib import check, ptr, stream_ptr
+from ._lib import call, ptr
 
 
 # --------------------------------------------------------------------------------- enums
@@ -50,9 +51,11 @@ class MeshInfo3D:
     def __init__(self, NZ: int, NY: int, NX: int, LZ: float, LY: float, LX: float):
         self._N = (int(NZ), int(NY), int(NX))
         self._L = tuple(float(np.float32(v)) for v in (LZ, LY, LX))
-        with np.errstate(divide="ignore", invalid="ignore"):
-            self._h = tuple(float(np.float32(np.float32(L) / np.float32(N - 1)))
-                            for N, L in zip(self._N, self._L))
+        if min(self._N) > 1:
+            self._h = tuple(float(np.float32(L) / np.float32(N - 1)) for N, L in zip(self._N, self._L))
+        else:  # a single node: L / 0 as float32 has it
+            with np.errstate(divide="ignore", invalid="ignore"):
+                self._h = tuple(float(np.float32(L) / np.float32(N - 1)) for N, L in zip(self._N, self._L))
 
     def getNZ(self): return self._N[0]
     def getNY(self): return self._N[1]
@@ -72,21 +75,20 @@ class MeshInfo3D:
 
 
 # ------------------------------------------------------------------------------- helpers
-def _op(name: str, t: torch.Tensor):
-    """The entry point for the tensor's value type: float32 -> name, float64 -> name_f64 (the
-    reference dispatched both, AT_DISPATCH_FLOATING_TYPES)."""
-    return getattr(_lib.lib(), name + ("_f64" if t.dtype == torch.float64 else ""))
+_TYPES = (torch.float32, torch.float64)
 
 
 def _check_input(t: torch.Tensor, name: str) -> None:
     """CHECK_INPUT of coreDefines.h:10-12, plus the float32 / float64 requirement."""
+    if type(t) is torch.Tensor and t.is_cuda and t.is_contiguous() and t.dtype in _TYPES:
+        return
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
     if t.device.type != "cuda":
         raise RuntimeError(f"{name} must be a CUDA tensor")
     if not t.is_contiguous():
         raise RuntimeError(f"{name} must be contiguous")
-    if t.dtype not in (torch.float32, torch.float64):
+    if t.dtype not in _TYPES:
         raise RuntimeError(f"{name} must be float32 or float64 (got {t.dtype})")
 
 
@@ -117,18 +119,14 @@ class Nabla3D_CD:
         nz, ny, nx = b.shape[:3]
         out = torch.empty(tuple(b.shape) + (3,), dtype=b.dtype, device=b.device)
         hz, hy, hx = self._mesh.h()
-        with torch.cuda.device(b.device):
-            check(_op("svs_nabla3d_forward", b)(ptr(b), nz, ny, nx, C, hz, hy, hx, self._bdry,
-                                                 ptr(out), stream_ptr(b.device)))
+        call("svs_nabla3d_forward", b, ptr(b), nz, ny, nx, C, hz, hy, hx, self._bdry, ptr(out))
         return out
 
     def _bwd(self, p, C):
         nz, ny, nx = p.shape[:3]
         out = torch.empty(tuple(p.shape[:-1]), dtype=p.dtype, device=p.device)
         hz, hy, hx = self._mesh.h()
-        with torch.cuda.device(p.device):
-            check(_op("svs_nabla3d_backward", p)(ptr(p), nz, ny, nx, C, hz, hy, hx, self._bdry,
-                                                  ptr(out), stream_ptr(p.device)))
+        call("svs_nabla3d_backward", p, ptr(p), nz, ny, nx, C, hz, hy, hx, self._bdry, ptr(out))
         return out
 
     def forward(self, b: torch.Tensor) -> torch.Tensor:
@@ -172,9 +170,8 @@ class AnisotropicNabla3D:
         sh = tuple(g.shape[:3])
         s = torch.empty(sh, dtype=g.dtype, device=g.device)
         n, t1, t2 = (torch.empty(sh + (3,), dtype=g.dtype, device=g.device) for _ in range(3))
-        with torch.cuda.device(g.device):
-            check(_op("svs_aniso3d_tangents", g)(ptr(g), int(np.prod(sh)), self._alpha, self._beta,
-                                                  ptr(s), ptr(n), ptr(t1), ptr(t2), stream_ptr(g.device)))
+        call("svs_aniso3d_tangents", g, ptr(g), math.prod(sh), self._alpha, self._beta, ptr(s), ptr(n), ptr(t1),
+             ptr(t2))
         return [s, n, t1, t2]
 
     def forwardVectorField(self, b, scalars, normals, tangents1, tangents2):
@@ -182,14 +179,13 @@ class AnisotropicNabla3D:
                       (tangents2, "tangents2")):
             _check_input(t, nm)
         _check_dim(b, 5)
-        nvox = int(np.prod(b.shape[:3]))
+        nvox = math.prod(b.shape[:3])
         if scalars.numel() < nvox or normals.numel() < 3 * nvox or tangents1.numel() < 3 * nvox:
             raise RuntimeError("tangent fields are smaller than the input field")
         _same_device(b, scalars, normals, tangents1, tangents2)
         out = torch.empty_like(b)
-        with torch.cuda.device(b.device):
-            check(_op("svs_aniso3d_apply", b)(ptr(b), nvox, ptr(scalars), ptr(normals), ptr(tangents1),
-                                               ptr(tangents2), ptr(out), stream_ptr(b.device)))
+        call("svs_aniso3d_apply", b, ptr(b), nvox, ptr(scalars), ptr(normals), ptr(tangents1), ptr(tangents2),
+             ptr(out))
         return out
 
     # The reference's backward is the same kernel (anisotropicDifferentialOps.h:437-444): D is
@@ -213,9 +209,7 @@ class Warping3D:
         _same_device(u, phi)
         out = torch.empty_like(u)
         hz, hy, hx = self._mesh.h()
-        with torch.cuda.device(u.device):
-            check(_op("svs_warp3d", u)(ptr(u), nz, ny, nx, C, ptr(phi), hz, hy, hx, self._interp,
-                                        self._bdry, ptr(out), stream_ptr(u.device)))
+        call("svs_warp3d", u, ptr(u), nz, ny, nx, C, ptr(phi), hz, hy, hx, self._interp, self._bdry, ptr(out))
         return out
 
     def forward(self, u: torch.Tensor, phi: torch.Tensor) -> torch.Tensor:
@@ -245,10 +239,8 @@ class Warping3D:
         gu = torch.empty_like(u)
         gp = torch.empty_like(phi)
         hz, hy, hx = self._mesh.h()
-        with torch.cuda.device(u.device):
-            check(_op("svs_warp3d_backward", u)(ptr(u), nz, ny, nx, ptr(phi), ptr(forward_out), hz, hy,
-                                                 hx, self._interp, self._bdry, ptr(gu), ptr(gp),
-                                                 stream_ptr(u.device)))
+        call("svs_warp3d_backward", u, ptr(u), nz, ny, nx, ptr(phi), ptr(forward_out), hz, hy, hx, self._interp,
+             self._bdry, ptr(gu), ptr(gp))
         return [gu, gp]
 
 
@@ -260,7 +252,8 @@ class WarpingCNN3D:
         self._interp = int(interpolation)
         self._bdry = int(boundary)
 
-    def forward(self, u: torch.Tensor, phi: torch.Tensor) -> torch.Tensor:
+    def forward(self, u: torch.Tensor, phi: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
+        """u warped by phi; into `out` where given (contiguous, of u's shape, type and device)."""
         _check_input(u, "u")
         _check_input(phi, "phi")
         _check_dim(u, 5)
@@ -269,11 +262,10 @@ class WarpingCNN3D:
         if tuple(phi.shape) != (B, nz, ny, nx, 3):
             raise RuntimeError("phi must have shape [B,NZ,NY,NX,3] matching u")
         _same_device(u, phi)
-        out = torch.empty_like(u)
+        if out is None:
+            out = torch.empty_like(u)
         hz, hy, hx = self._mesh.h()
-        with torch.cuda.device(u.device):
-            check(_op("svs_warp_cnn3d", u)(ptr(u), B, C, nz, ny, nx, ptr(phi), hz, hy, hx, self._interp,
-                                            self._bdry, ptr(out), stream_ptr(u.device)))
+        call("svs_warp_cnn3d", u, ptr(u), B, C, nz, ny, nx, ptr(phi), hz, hy, hx, self._interp, self._bdry, ptr(out))
         return out
 
 
@@ -290,16 +282,14 @@ class Prolongation3D:
 
     def _run(self, u, tail, out_components=None):
         nz, ny, nx = u.shape[:3]
-        C = int(np.prod(tail)) if tail else 1
+        C = math.prod(tail) if tail else 1
         d = self._dst
         tz, ty, tx = d.getNZ(), d.getNY(), d.getNX()
         co = C if out_components is None else int(out_components)
         out = torch.empty((tz, ty, tx) + (tuple(tail) if out_components is None else (co,)), dtype=u.dtype, device=u.device)
         s = self._src
-        with torch.cuda.device(u.device):
-            check(_op("svs_prolongate3d_padded", u)(ptr(u), nz, ny, nx, C, s.getLZ(), s.getLY(), s.getLX(),
-                                                     tz, ty, tx, d.getLZ(), d.getLY(), d.getLX(), self._interp,
-                                                     self._bdry, co, ptr(out), stream_ptr(u.device)))
+        call("svs_prolongate3d_padded", u, ptr(u), nz, ny, nx, C, s.getLZ(), s.getLY(), s.getLX(), tz, ty, tx,
+             d.getLZ(), d.getLY(), d.getLX(), self._interp, self._bdry, co, ptr(out))
         return out
 
     def forward(self, u: torch.Tensor) -> torch.Tensor:
@@ -343,11 +333,8 @@ def TVL1OF3D_proxPrimal(primalVariable: torch.Tensor, primalStepSize_tau: float,
         raise RuntimeError("proxPrimal: tensor sizes do not match the mesh")
     _same_device(primalVariable, rho, I1_warped_grad)
     out = torch.empty_like(primalVariable)
-    dev = primalVariable.device
-    with torch.cuda.device(dev):
-        check(_op("svs_tvl1_prox_primal", primalVariable)(ptr(primalVariable), n, float(primalStepSize_tau),
-                                              float(primalFctWeight_Matching), ptr(rho), ptr(I1_warped_grad),
-                                              ptr(out), stream_ptr(dev)))
+    call("svs_tvl1_prox_primal", primalVariable, ptr(primalVariable), n, float(primalStepSize_tau),
+         float(primalFctWeight_Matching), ptr(rho), ptr(I1_warped_grad), ptr(out))
     return out
 
 
@@ -361,10 +348,8 @@ def TVL1OF3D_proxDual(dualVariable: torch.Tensor, dualStepSize_sigma: float, dua
     if dualVariable.numel() != 9 * n:
         raise RuntimeError("proxDual: tensor size does not match the mesh")
     out = torch.empty_like(dualVariable)
-    dev = dualVariable.device
-    with torch.cuda.device(dev):
-        check(_op("svs_tvl1_prox_dual", dualVariable)(ptr(dualVariable), n, float(dualStepSize_sigma),
-                                            float(dualFctWeight_TV), ptr(out), stream_ptr(dev)))
+    call("svs_tvl1_prox_dual", dualVariable, ptr(dualVariable), n, float(dualStepSize_sigma),
+         float(dualFctWeight_TV), ptr(out))
     return out
 
 

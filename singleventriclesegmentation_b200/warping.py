@@ -13,7 +13,9 @@ from typing import Tuple
 
 import torch
 
+from . import _lib
 from . import opticalFlow
+from ._lib import ptr
 from .flow_utils import get_interpolation_type, get_mesh_length
 
 
@@ -26,12 +28,36 @@ class Warp:
         self.mesh_length_type = mesh_length_type
         self.LZ, self.LY, self.LX = lenghts
 
+    def op(self, shape) -> opticalFlow.WarpingCNN3D:
+        """The operator for volumes of `shape` = (Z, Y, X)."""
+        LZ, LY, LX = get_mesh_length(self.mesh_length_type, *shape, self.LZ, self.LY, self.LX)
+        return opticalFlow.WarpingCNN3D(opticalFlow.MeshInfo3D(*shape, LZ, LY, LX), self.interpolation, self.boundary)
+
     def __call__(self, x: torch.Tensor, u: torch.Tensor) -> torch.Tensor:
-        NZ, NY, NX = x.shape[2:]
-        LZ, LY, LX = get_mesh_length(self.mesh_length_type, NZ, NY, NX, self.LZ, self.LY, self.LX)
-        mesh_info = opticalFlow.MeshInfo3D(NZ, NY, NX, LZ, LY, LX)
-        op = opticalFlow.WarpingCNN3D(mesh_info, self.interpolation, self.boundary)
-        return op.forward(x.contiguous(), u.contiguous())
+        return self.op(x.shape[2:]).forward(x.contiguous(), u.contiguous())
+
+
+def _propagate_native(warp: Warp, initial_mask, final_mask, forward_flow, backward_flow):
+    """Both chains in one native call, or None where the inputs ask for the step-by-step form."""
+    ts = (initial_mask, final_mask, forward_flow, backward_flow)
+    if type(warp) is not Warp or torch.get_default_dtype() != torch.float32:
+        return None
+    if not all(type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and t.device == ts[0].device for t in ts):
+        return None
+    Z, Y, X = shape = tuple(initial_mask.shape[2:])
+    T = forward_flow.shape[0]
+    if (initial_mask.dim() != 5 or tuple(initial_mask.shape[:2]) != (1, 1) or final_mask.shape != initial_mask.shape
+            or tuple(forward_flow.shape) != (T, Z, Y, X, 3) or backward_flow.shape != forward_flow.shape
+            or not (forward_flow.is_contiguous() and backward_flow.is_contiguous())
+            or Z > 65535 or not 0 < Z * Y * X < 2 ** 31 - 1):
+        return None
+    first, last = initial_mask.contiguous(), final_mask.contiguous()
+    scratch = torch.empty((4,) + shape, dtype=torch.float32, device=first.device)
+    fwd, bwd = (torch.empty((T + 1, 1) + shape, dtype=torch.float32, device=first.device) for _ in range(2))
+    op = warp.op(shape)
+    _lib.call("svs_propagate_masks3d", first, ptr(first), ptr(last), ptr(forward_flow), ptr(backward_flow), T, Z, Y, X,
+              *op._mesh.h(), op._interp, op._bdry, ptr(scratch), ptr(fwd), ptr(bwd))
+    return fwd, bwd
 
 
 def propagate(warp: Warp, initial_mask: torch.Tensor, final_mask: torch.Tensor,
@@ -39,6 +65,9 @@ def propagate(warp: Warp, initial_mask: torch.Tensor, final_mask: torch.Tensor,
     """warping.py:205-243: chain the float masks through the flows both ways, reverse the
     backward chain, then threshold at 0.5. Masks [1,1,Z,Y,X]; flows [T-1,Z,Y,X,3]."""
     assert forward_flow.shape[0] == backward_flow.shape[0], "Forward and backward flow have different timesteps"
+    both = _propagate_native(warp, initial_mask, final_mask, forward_flow, backward_flow)
+    if both is not None:
+        return both
     fwd = [initial_mask]
     bwd = [final_mask]
     for t in range(forward_flow.shape[0]):
@@ -54,6 +83,13 @@ def propagate_batched(warp: Warp, masks: torch.Tensor, flows: torch.Tensor) -> t
     """Many independent chains at once: masks [K,1,Z,Y,X] are warped step by step with flows
     [T-1,K,Z,Y,X,3] (chain k uses flows[:, k]); one batched launch per step instead of one per
     chain. Returns the float chains [T,K,1,Z,Y,X] (not thresholded)."""
+    if type(warp) is Warp and type(masks) is torch.Tensor and masks.is_cuda and masks.dim() == 5 and not masks.requires_grad:
+        op = warp.op(masks.shape[2:])  # every step straight into its place of the result
+        out = masks.new_empty((flows.shape[0] + 1,) + tuple(masks.shape))
+        out[0].copy_(masks)
+        for t in range(flows.shape[0]):
+            op.forward(out[t], flows[t].contiguous(), out[t + 1])
+        return out
     out = [masks]
     for t in range(flows.shape[0]):
         out.append(warp(out[-1], flows[t]))
