@@ -1004,21 +1004,38 @@ class ResidentTurn {
 };
 
 // Modelled microseconds per iteration, fitted to measurements on one B200.
-// The per-iteration kernels over a level's voxels (2-byte fields, 80^3 pairs: 20.3 us for one, 54
-// for 4, 142 for 12, 670 for 68; f32: 20.5 for one, 72 for 4): launch and ramp, bandwidth, and the
-// unfilled last wave of a small batch.
-double stream_us(int storage, double voxels) {
-  if (voxels <= 0.0) return 0.0;
-  return 10.0 + voxels * (storage == SVS_STORAGE_F32 ? 28e-6 : 19.3e-6) + std::min(14.0, 1.6e-6 * voxels);
+// The per-iteration kernels: what each pair's column tiles cost on a full GPU (the least of the
+// automatic variants, auto_choice), more where a batch leaves waves part-empty or runs as groups of
+// several variants, and launch and ramp. 80^3 pairs, 2-byte fields: 20 us for one, 54 for 4, 142 for
+// 12, 670 for 68; f32 20.5 for one, 72 for 4; 96^3 31, 120x104x128 53, eight uneven volumes 138.
+double stream_pair_us(int storage, const Desc& d, int* variant) {
+  if (storage == SVS_STORAGE_F32) {
+    *variant = 0;
+    return 1e-3 * 12.1 * ceil_div(d.nx, 32) * ceil_div(d.ny, 16) * d.nz;
+  }
+  double best = -1.0;
+  for (const AutoCost& c : kAutoCosts16) {
+    const TileShape& ts = kTileShapes[c.tid - 1];
+    const double us = 1e-3 * c.ns * ceil_div(d.nx, ts.tx) * ceil_div(d.ny, ts.ty) * d.nz;
+    if (best < 0 || us < best) {
+      best = us;
+      *variant = c.tid;
+    }
+  }
+  return best;
+}
+double stream_us(double work, bool groups) {
+  return work <= 0.0 ? 0.0 : (10.0 + work * (1.0 + 0.25 / (1.0 + work / 100.0))) * (groups ? 1.15 : 1.0);
 }
 // A resident launch with boxes of `threads` threads of `np` voxel pairs and `words` face words:
-// the two exchanges (2.5 us with next to no work), the warps' pairs, the words' traffic. 6x6x6
-// boxes 2.7 us, 8x8x10 3.4, 10x10x10 4.1 (np 1), 20x8x8 4.6, 20x10x10 6.1 (np 2; f32 5.3 and 6.9),
-// 16x12x20 10.6 (np 5; f32 14.6).
-float resident_us(int storage, int np, int threads, int words) {
+// the two exchanges (2.5 us with next to no work), the warps' pairs, the words' traffic, and the
+// launch itself over its iterations. 6x6x6 boxes 2.7 us, 8x8x10 3.4, 10x10x10 4.0 (np 1), 20x8x8
+// 4.6, 40x8x6 5.8, 20x10x10 6.2 (np 2; f32 5.3, 6.4 and 6.8), 20x12x15 9.7, 16x12x20 10.5 (np 5;
+// f32 14.2 and 14.6).
+float resident_us(int storage, int np, int threads, int words, int iters) {
   const bool f32 = storage == SVS_STORAGE_F32;
   const float pair_us = np > 2 ? (f32 ? 0.19f : 0.12f) : np == 2 && f32 ? 0.11f : 0.085f;
-  return 2.45f + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words;
+  return 2.45f + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words + 6.0f / iters;
 }
 
 // ---- resident iterations (svs_resident.cuh): which pairs of a level, in which boxes
@@ -1027,7 +1044,7 @@ struct ResBoxes {
   float us;  // modelled time per iteration
 };
 // Boxes that fit a compiled shape, by modelled time: x in pairs, z in whole groups of NP pairs.
-std::vector<ResBoxes> resident_boxes(int storage, const ResCaps& c) {
+std::vector<ResBoxes> resident_boxes(int storage, int iters, const ResCaps& c) {
   std::vector<ResBoxes> out;
   for (int bx = 4; bx <= 64; bx += 2)
     for (int by = 2; by <= 48; ++by)
@@ -1039,7 +1056,7 @@ std::vector<ResBoxes> resident_boxes(int storage, const ResCaps& c) {
         const int col = 2 * bz * by;
         if ((bz + 2) * (by + 2) * bx + col > c.cu || std::max(bz * by * bx + col, std::max(bz * (by + 2) * bx, (bz + 2) * by * bx)) > c.cq)
           continue;
-        out.push_back({bx, by, bz, threads, words, resident_us(storage, c.np, threads, words)});
+        out.push_back({bx, by, bz, threads, words, resident_us(storage, c.np, threads, words, iters)});
       }
   std::sort(out.begin(), out.end(), [](const ResBoxes& a, const ResBoxes& b) { return a.us < b.us; });
   return out;
@@ -1080,19 +1097,33 @@ void plan_resident(svs_plan& P, int level) {
     float us;
     int count, box;
   };
-  double best_us = -1.0, all_vox = 0.0;
+  double best_us = -1.0;
   int best_shape = -1;
   std::vector<int> best_box;
   std::vector<std::vector<ResBoxes>> boxes(kResShapes);
-  for (int i = 0; i < np; ++i) all_vox += (double)D[i].n;
+  std::vector<double> work(np);
+  std::vector<int> variant(np);
+  for (int i = 0; i < np; ++i) work[i] = stream_pair_us(P.prm.storage, D[i], &variant[i]);
+  // time of the per-iteration launches of the pairs for which pick[i] < 0
+  auto streamed = [&](const std::vector<int>& pick) {
+    double w = 0.0;
+    int first = -1;
+    bool groups = false;
+    for (int i = 0; i < np; ++i) {
+      if (pick[i] >= 0) continue;
+      w += work[i];
+      if (first < 0) first = variant[i];
+      groups = groups || variant[i] != first;
+    }
+    return stream_us(w, groups);
+  };
   for (int sh = 0; sh < kResShapes; ++sh) {
     int occ = 0;
     if (!resident_variant(P.prm.storage, sh, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, &occ)) continue;
-    boxes[sh] = resident_boxes(P.prm.storage, kResCaps[sh]);
+    boxes[sh] = resident_boxes(P.prm.storage, P.prm.max_outer_iterations, kResCaps[sh]);
     // per pair: fewer boxes for more time
     std::vector<std::vector<Choice>> front(np);
     std::vector<float> bounds;
-    double vox = 0.0;
     for (int i = 0; i < np; ++i) {
       if (!resident_ok(P, D[i])) continue;
       int same = -1;
@@ -1110,7 +1141,6 @@ void plan_resident(svs_plan& P, int level) {
           bounds.push_back(boxes[sh][b].us);
         }
       }
-      if (!front[i].empty()) vox += (double)D[i].n;
     }
     std::sort(bounds.begin(), bounds.end());
     bounds.erase(std::unique(bounds.begin(), bounds.end()), bounds.end());
@@ -1136,9 +1166,8 @@ void plan_resident(svs_plan& P, int level) {
         longest = std::max(longest, c->us);
       }
       total += longest;
-      // the pairs left out keep the per-iteration launches
-      if (!ok || vox == 0.0) continue;
-      total += stream_us(P.prm.storage, all_vox - vox);
+      if (!ok) continue;
+      total += streamed(pick);  // the pairs left out
       if (best_us < 0 || total < best_us) {
         best_us = total;
         best_shape = sh;
@@ -1146,7 +1175,7 @@ void plan_resident(svs_plan& P, int level) {
       }
     }
   }
-  if (best_us < 0 || best_us >= stream_us(P.prm.storage, all_vox)) return;
+  if (best_us < 0 || best_us >= streamed(std::vector<int>(np, -1))) return;
   svs_plan::ResStep st;
   int npairs = 0;
   auto flush = [&] {
