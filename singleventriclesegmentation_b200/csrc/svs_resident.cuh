@@ -27,11 +27,11 @@
 //
 // Measured on one B200 (us per iteration; before: one launch per iteration, march along z):
 //   f16-flow32 80^3 10.6 (20.4), 48^3 3.4 (14.4), 40^3 3.3 (10.3), 20^3 2.8 (8.2);
-//   f32 80^3 14.6 (20.5), 48^3 3.4 (12.3), 20^3 2.8 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
+//   f32 80^3 13.8 (20.5), 48^3 3.4 (12.3), 20^3 2.8 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
 // Small boxes are bound by the two exchanges (about 2.5 us: publish, poll, barriers). 80^3 is
 // bound by the latency of 12 warps of 168 registers (about 8,000 cycles of dual, 5,800 of primal)
 // and by the words' L2 traffic (3.6 MB per exchange each way). Its f32 form keeps p alone (90
-// registers of 168, 400 bytes spilled) and reads D (12 MB) and rho_c, gw (8 MB) from L2 in every
+// registers of 168, 350 bytes spilled) and reads D (12 MB) and rho_c, gw (8 MB) from L2 in every
 // iteration; reading D one pair ahead took 15.5 us (12 more registers), 8 pairs by 256 threads 21.5.
 //
 // Boundaries (MIRROR with power-of-two 0.5/h only, see resident_ok in svs_solver.cu): central
@@ -76,12 +76,14 @@ struct ResidentArgs {
 // Compiled shapes: NP voxel pairs per thread, up to NT threads; CU floats per component of u (with
 // its halo planes, rows and columns) and CQ of each of q_x (halo columns), q_y (halo rows) and
 // q_z (halo planes); up to NE face voxels per thread. KEEP_D, KEEP_R: the tensor, and rho_c and
-// the warped gradient, stay in registers; else they are read again in every iteration, D one pair
-// ahead of its use, the others before the wait for q's halo.
+// the warped gradient, stay in registers; else they are read again in every iteration, D where it
+// is used, the others before the wait for q's halo. ROLL: the primal keeps q_z of two planes from pair
+// to pair instead of reading each plane twice. Taken where p alone is held (f32 80^3 14.7 -> 13.8 us
+// per iteration); with D held too it takes registers that are not there (f16-flow32 80^3 10.6 -> 10.8).
 template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_D_, bool KEEP_R_>
 struct ResShape {
   static constexpr int NP = NP_, NT = NT_, CU = CU_, CQ = CQ_, NE = NE_;
-  static constexpr bool KEEP_D = KEEP_D_, KEEP_R = KEEP_R_;
+  static constexpr bool KEEP_D = KEEP_D_, KEEP_R = KEEP_R_, ROLL = !KEEP_D;
   // the register file holds 16,384 registers per scheduler, a quarter of the warps each
   static constexpr int WARPS = (NT + 31) / 32, MAXREG = 16384 / ((WARPS + 3) / 4 * 32) / 8 * 8;
   static constexpr int REGS = MAXREG > 255 ? 255 : MAXREG;
@@ -437,9 +439,18 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
     }
     // ---- primal
     asm volatile("" : "+r"(iu), "+r"(iqx), "+r"(aL), "+r"(aR));
+    float2 zm[3], zc[3];  // ROLL: q_z of the planes below and at the pair's
+    if (C::ROLL && nj > 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        zm[c] = pair_at(sqz + c * C::CQ + iqx);
+        zc[c] = pair_at(sqz + c * C::CQ + iqx + PX);
+      }
+    }
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
-      if (j < nj) {
+      // (ROLL: planes past the box's last are computed, on cells inside the arrays, and not stored)
+      if (C::ROLL ? nj > 0 : j < nj) {
         float2 uo[3], g[3], n[3], dv[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -456,14 +467,19 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
           const float2 dx = vsub(make_float2(qx[xlo ? aL - dUQ + j * by : iqx + j * PX - 1], o.x),
                                  make_float2(o.y, qx[xhi ? aR - dUQ + j * by : iqx + j * PX + 2]));
           const float2 dy = vsub(pair_at(qy - bx), pair_at(qy + bx));
-          const float2 dz = vsub(pair_at(qz - PX), pair_at(qz + PX));
-          dv[c] = sum3(dx, dy, dz);
+          const float2 zp = pair_at(qz + PX);
+          dv[c] = sum3(dx, dy, vsub(C::ROLL ? zm[c] : pair_at(qz - PX), zp));
+          if constexpr (C::ROLL) {
+            zm[c] = zc[c];
+            zc[c] = zp;
+          }
         }
         primal_apply(uo, dv, 0.5f * tau, t, g, n);
         // (the voxel beside the volume's last one, odd nx: a mirror cell, filled again below)
+        if (!C::ROLL || j < nj)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          *reinterpret_cast<float2*>(su + c * C::CU + iu + j * PU) = as_stored<SU>(n[c]);
+          for (int c = 0; c < 3; ++c)
+            *reinterpret_cast<float2*>(su + c * C::CU + iu + j * PU) = as_stored<SU>(n[c]);
       }
     }
     if (it + 1 < a.iters) {

@@ -1034,7 +1034,7 @@ double stream_us(double work, bool groups) {
 // f32 14.2 and 14.6).
 float resident_us(int storage, int np, int threads, int words, int iters) {
   const bool f32 = storage == SVS_STORAGE_F32;
-  const float pair_us = np > 2 ? (f32 ? 0.19f : 0.12f) : np == 2 && f32 ? 0.11f : 0.085f;
+  const float pair_us = np > 2 ? (f32 ? 0.175f : 0.12f) : np == 2 && f32 ? 0.11f : 0.085f;
   return 2.45f + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words + 6.0f / iters;
 }
 
