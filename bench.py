@@ -271,11 +271,12 @@ def config_dict(args, storage):
 
 # ------------------------------------------------------------------------ shared helpers
 def tune_plan(plan, storage: str, levels: int = 3, per_class: bool = False):
-    """Pick the fastest iterate-kernel variant per pyramid level on the plan's own state (TMA
-    and split-role forms); with per_class also per size class of each level."""
+    """Pick the fastest iterate-kernel variant per pyramid level on the plan's own state (the
+    automatic choice, which may keep iterations on the chip, TMA and split-role forms); with
+    per_class also per size class of each level."""
     from singleventriclesegmentation_b200 import _lib, autotune
     n = int(_lib.lib().svs_tvl1_num_tiles())
-    cands = [t for t in range(1, n + 1) if _lib.tile_info(t)["form"] != "plain"]
+    cands = [0] + [t for t in range(1, n + 1) if _lib.tile_info(t)["form"] != "plain"]
     return autotune.tune(plan, storage, levels, candidates=cands, use_cache=False, iters=12, per_class=per_class)
 
 
@@ -799,7 +800,7 @@ def main():
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
             "dtype": "f32" if args.storage == "f32" else f"f32 math, {args.storage} storage",
-            "level_tiles": plan.level_tiles()[:3],
+            "level_tiles": plan.level_tiles()[:3], "level_resident": [plan.level_resident(l) for l in range(3)],
             "data": "synthetic", "config": config_dict(args, args.storage),
             "e2e": {"value": e2e_value, "unit": "pairs/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": int(launches),

@@ -1,6 +1,8 @@
 """Autotuner for the fused iterate kernel: picks, per pyramid level of a plan, the kernel variant
 (TMA pipeline or plain-load form, tile shape, prefetch distance) with the shortest measured time
-on the plan's own state, and caches the choice on disk.
+on the plan's own state, and caches the choice on disk. Variant 0 is the plan's automatic choice:
+the only one under which iterations stay on the chip (any explicit variant means one launch per
+iteration).
 
 The variants are listed in include/svsflow.h (svs_tvl1_plan_set_tile). A level's "size class" is
 the multiset of its volume sizes; the cache key is (GPU name, storage, level sizes).
@@ -21,6 +23,13 @@ from .tvl13d import SolverPlan
 CACHE = os.environ.get("SVS_AUTOTUNE_CACHE", os.path.join(os.path.expanduser("~"), ".cache", "svsflow", "autotune.json"))
 
 
+# An explicit variant replaces the automatic choice when it takes less than this part of its time. These
+# short timings do not reach the power cap that a long solve of streaming launches runs at, while
+# iterations on the chip stay below it: 68 pairs of 80^3 with FP32 storage timed 0.95 ms per
+# iteration with variant 13 and 1.0 ms automatically, but solved in 5.39 s and 5.20 s (1.66 and 1.97 GHz).
+AUTO_MARGIN = 0.92
+
+
 def _level_dims(dims: Sequence[Tuple[int, int, int]], levels: int) -> List[List[Tuple[int, int, int]]]:
     out = []
     cur = [tuple(d) for d in dims]
@@ -33,7 +42,7 @@ def _level_dims(dims: Sequence[Tuple[int, int, int]], levels: int) -> List[List[
 def _variants_signature() -> str:
     """The compiled variant table, so that a cache written by another build is not reused."""
     n = int(_lib.lib().svs_tvl1_num_tiles())
-    return ",".join("{tx}x{ty}/{dist}{f}{lane_voxels}".format(f=i["form"][0], **i)
+    return "auto," + ",".join("{tx}x{ty}/{dist}{f}{lane_voxels}".format(f=i["form"][0], **i)
                     for i in map(_lib.tile_info, range(1, n + 1)))
 
 
@@ -60,6 +69,13 @@ def _store(db: Dict[str, int]) -> None:
         os.replace(tmp, CACHE)
     except OSError:
         pass
+
+
+def _iters(plan: SolverPlan, tile: int, iters: int) -> int:
+    """Iterations to time `tile` over: a warp's for the automatic choice, whose launches may each run
+    all of a warp's iterations. Their start (20 to 30 us for each launch of up to 148 boxes) is part
+    of a warp's time, and over 12 iterations it would count 25 times as much."""
+    return iters if tile else max(iters, int(plan.params.max_outer_iterations))
 
 
 def time_variant(plan: SolverPlan, level: int, tile: int, iters: int = 6) -> Optional[float]:
@@ -141,7 +157,7 @@ def tune(plan: SolverPlan, storage: str, levels: int, candidates: Optional[Seque
     """Choose and set the fastest variant per level; returns the chosen ids (level 0 first).
     With per_class, then let each size class of a level take one of the level's
     `class_candidates` fastest variants (tune_classes)."""
-    candidates = list(candidates or range(1, int(_lib.lib().svs_tvl1_num_tiles()) + 1))
+    candidates = list(candidates or range(0, int(_lib.lib().svs_tvl1_num_tiles()) + 1))
     db = _load() if use_cache else {}
     chosen = []
     lds = _level_dims(plan.dims, levels)
@@ -150,16 +166,16 @@ def tune(plan: SolverPlan, storage: str, levels: int, candidates: Optional[Seque
         best = db.get(key)
         ranked = None
         if best is None or per_class:
-            timings = {t: time_variant(plan, level, t, iters) for t in candidates}
+            timings = {t: time_variant(plan, level, t, _iters(plan, t, iters)) for t in candidates}
             timings = {t: v for t, v in timings.items() if v is not None}
-            ranked = sorted(timings, key=timings.get)
+            ranked = sorted(timings, key=lambda t: timings[t] * (1.0 if t else AUTO_MARGIN))
             best = ranked[0] if best is None else best
             db[key] = best
         plan.set_level_tile(level, best)
         chosen.append(best)
         if per_class and ranked:
-            cls = tune_classes(plan, level, [t for t in ranked[:class_candidates + 1] if t != best][:class_candidates],
-                               iters)
+            cls = tune_classes(plan, level, [t for t in ranked[:class_candidates + 1] if t and t != best][:class_candidates],
+                               _iters(plan, best, iters))
             plan.class_tiles = getattr(plan, "class_tiles", {})
             plan.class_tiles[level] = cls
     if use_cache:
