@@ -25,9 +25,17 @@
 // from tag 0. Polling is bounded (ResidentArgs::wait_us); a box that gives up raises the abort
 // word, which ends its neighbours' waits and the plan's later launches.
 //
+// CLUSTER: a volume of at most 16 boxes runs in one thread-block cluster instead. The faces are then
+// written straight into the halo cells of the neighbours' shared memory, and one cluster barrier
+// per exchange replaces words, tags and polling (every box has read its halo before it sends what
+// lets a neighbour write again: the same order as above). No box of another pair is waited for, so the
+// launch is not cooperative. An exchange takes about 0.75 us instead of 1.25: 20^3 2.8 -> 2.3 us per iteration (16 boxes
+// of 10x10x5), 9x11x12 2.7 -> 1.8. From about 250 voxel pairs per box on, the boxes' arithmetic is worth more
+// than that (24^3: 3.2 us in one cluster, 2.7 us on 144 SMs), and the choice below sees it.
+//
 // Measured on one B200 (us per iteration; before: one launch per iteration, march along z):
-//   f16-flow32 80^3 10.6 (20.4), 48^3 3.4 (14.4), 40^3 3.3 (10.3), 20^3 2.8 (8.2);
-//   f32 80^3 13.8 (20.5), 48^3 3.4 (12.3), 20^3 2.8 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
+//   f16-flow32 80^3 10.6 (20.4), 48^3 3.4 (14.4), 40^3 3.3 (10.3), 20^3 2.3 (8.2);
+//   f32 80^3 13.8 (20.5), 48^3 3.4 (12.3), 20^3 2.3 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
 // Small boxes are bound by the two exchanges (about 2.5 us: publish, poll, barriers). 80^3 is
 // bound by the latency of 12 warps of 168 registers (about 8,000 cycles of dual, 5,800 of primal)
 // and by the words' L2 traffic (3.6 MB per exchange each way). Its f32 form keeps p alone (90
@@ -59,6 +67,7 @@ struct ResPair {
 struct ResLaunch {
   ResPair pair[kResSlots];
   unsigned char of[kResSlots];  // pair of each block
+  int cluster;                  // CLUSTER shapes: blocks per cluster (a pair each), else 0
 };
 
 struct ResidentArgs {
@@ -80,9 +89,10 @@ struct ResidentArgs {
 // is used, the others before the wait for q's halo. ROLL: the primal keeps q_z of two planes from pair
 // to pair instead of reading each plane twice. Taken where p alone is held (f32 80^3 14.7 -> 13.8 us
 // per iteration); with D held too it takes registers that are not there (f16-flow32 80^3 10.6 -> 10.8).
-template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_D_, bool KEEP_R_>
+template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_D_, bool KEEP_R_, bool CLUSTER_ = false>
 struct ResShape {
   static constexpr int NP = NP_, NT = NT_, CU = CU_, CQ = CQ_, NE = NE_;
+  static constexpr bool CLUSTER = CLUSTER_;
   static constexpr bool KEEP_D = KEEP_D_, KEEP_R = KEEP_R_, ROLL = !KEEP_D;
   // the register file holds 16,384 registers per scheduler, a quarter of the warps each
   static constexpr int WARPS = (NT + 31) / 32, MAXREG = 16384 / ((WARPS + 3) / 4 * 32) / 8 * 8;
@@ -137,6 +147,19 @@ __device__ __forceinline__ uint4 word_poll(const uint4* p, unsigned on) {
       : "memory");
   return v;
 }
+// Shared memory of another CTA of the cluster, and the cluster's barrier (every thread of the cluster
+// that has not returned; what was written before it can be read after it).
+__device__ __forceinline__ unsigned peer_address(const void* p, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void peer_store(unsigned p, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 __device__ __forceinline__ float2 vsub(float2 a, float2 b) { return vadd(a, make_float2(-b.x, -b.y)); }
 
 template <typename SU, typename SP, typename C>
@@ -155,7 +178,12 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
   const ResPair& B = L.pair[L.of[blockIdx.x]];
   const Desc& d = descs[B.desc];
   // a stopped pair (the flag is the same in every box of the pair), or an earlier launch gave up
-  if (__syncthreads_or((d.stop && *d.stop) || *reinterpret_cast<volatile int*>(a.abort))) return;
+  if constexpr (C::CLUSTER) {
+    if (d.stop && *d.stop) return;
+    if (blockIdx.x - B.first >= B.gx * B.gy * B.gz) return;  // no box for this block of the cluster
+  } else {
+    if (__syncthreads_or((d.stop && *d.stop) || *reinterpret_cast<volatile int*>(a.abort))) return;
+  }
   const int bx = __shfl_sync(~0u, (int)B.bx, 0), by = __shfl_sync(~0u, (int)B.by, 0), bz = __shfl_sync(~0u, (int)B.bz, 0);
   const int box = blockIdx.x - B.first;
   const int gz_ = box / (B.gx * B.gy), gy_ = (box - gz_ * B.gx * B.gy) / B.gx, gx_ = box - (gz_ * B.gy + gy_) * B.gx;
@@ -181,6 +209,7 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
   const int S = a.words;
   unsigned ucell[C::NE], qcell[C::NE];  // halo | own << 16 (u's from 0, q's from sqx)
   int word[C::NE];                      // word to publish to (u), -1: volume face, -2: none
+  unsigned peer[C::CLUSTER ? C::NE : 1];  // CLUSTER: u of the neighbouring box (halo: its cells)
 #pragma unroll
   for (int i = 0; i < C::NE; ++i) {
     const int e = tid + i * nt;
@@ -231,6 +260,11 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       const int o = (z0 + vz) * gplane + (y0 + vy) * d.pitch + x0 + vx;
 #pragma unroll
       for (int c = 0; c < 3; ++c) su[c * C::CU + at(outside)] = Store<SU>::ld(u_src + (long long)c * cs + o);
+      if constexpr (C::CLUSTER) {
+        peer[i] = peer_address(su, (unsigned)(box + (hi ? step : -step)));
+        ucell[i] = at(hi ? -1 : n) | at(edge) << 16;
+        qcell[i] = q_at(hi ? -1 : n) | q_at(edge) << 16;
+      }
     } else {
       word[i] = -1;
       ucell[i] = at(outside) | at(hi ? m - 2 : 1) << 16;
@@ -318,7 +352,13 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
 #pragma unroll
     for (int i = 0; i < C::NE; ++i) {
       if (word[i] >= 0) {
-        word_publish(a.xbuf + word[i] + (q ? S : 0), v[i][0], v[i][1], v[i][2], tag);
+        if constexpr (C::CLUSTER) {
+          const unsigned out = peer[i] + 4 * ((q ? 3 * C::CU : 0) + ((q ? qcell[i] : ucell[i]) & 0xffff));
+#pragma unroll
+          for (int c = 0; c < 3; ++c) peer_store(out + 4 * c * st, v[i][c]);
+        } else {
+          word_publish(a.xbuf + word[i] + (q ? S : 0), v[i][0], v[i][1], v[i][2], tag);
+        }
       } else if (word[i] == -1) {
         float* out = s + (q ? qcell[i] >> 16 : ucell[i] & 0xffff);
         out[0] = q ? 0.f : v[i][0];
@@ -372,6 +412,7 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
 #pragma unroll
       for (int c = 0; c < 3; ++c) su[c * C::CU + (ucell[i] & 0xffff)] = su[c * C::CU + (ucell[i] >> 16)];
   __syncthreads();
+  if constexpr (C::CLUSTER) cluster_barrier();  // every box's arrays are filled before a neighbour writes to them
 
   bool bad = false;
   float next_sigma = __ldg(a.sig), next_tau = __ldg(a.tau);
@@ -432,10 +473,14 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
     }
     __syncthreads();
     send(true, (unsigned)it + 1);
-    bad = !receive(true, (unsigned)it + 1);
-    if (__syncthreads_or(bad)) {
-      bad = true;
-      break;
+    if constexpr (C::CLUSTER) {
+      cluster_barrier();
+    } else {
+      bad = !receive(true, (unsigned)it + 1);
+      if (__syncthreads_or(bad)) {
+        bad = true;
+        break;
+      }
     }
     // ---- primal
     asm volatile("" : "+r"(iu), "+r"(iqx), "+r"(aL), "+r"(aR));
@@ -485,10 +530,14 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
     if (it + 1 < a.iters) {
       __syncthreads();
       send(false, (unsigned)it + 1);
-      bad = !receive(false, (unsigned)it + 1);
-      if (__syncthreads_or(bad)) {
-        bad = true;
-        break;
+      if constexpr (C::CLUSTER) {
+        cluster_barrier();
+      } else {
+        bad = !receive(false, (unsigned)it + 1);
+        if (__syncthreads_or(bad)) {
+          bad = true;
+          break;
+        }
       }
     }
   }
@@ -522,11 +571,13 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       }
     }
   }
+  if constexpr (!C::CLUSTER) {
 #pragma unroll
-  for (int i = 0; i < C::NE; ++i) {
-    if (word[i] < 0) continue;
-    word_publish(const_cast<uint4*>(in0) + tid + i * nt, 0.f, 0.f, 0.f, 0u);
-    word_publish(const_cast<uint4*>(in0) + S + tid + i * nt, 0.f, 0.f, 0.f, 0u);
+    for (int i = 0; i < C::NE; ++i) {
+      if (word[i] < 0) continue;
+      word_publish(const_cast<uint4*>(in0) + tid + i * nt, 0.f, 0.f, 0.f, 0u);
+      word_publish(const_cast<uint4*>(in0) + S + tid + i * nt, 0.f, 0.f, 0.f, 0u);
+    }
   }
 }
 
@@ -536,16 +587,21 @@ using ResMid = ResShape<2, 512, 3456, 2688, 4, true, false>;
 // (5 pairs by 384 threads: 6 by 320 took 13.4 us at 80^3 f16-flow32, 8 by 256 11.9-14, against 10.6;
 // the register file is split by scheduler, so 13 to 16 warps would have 128 registers each)
 template <typename SP> using ResLarge = ResShape<5, 384, 5408, 4480, 4, sizeof(SP) == 2, false>;
-constexpr int kResShapes = 3, kResMaxWords = 2048;
+using ResCluster = ResShape<1, 512, 1920, 1408, 4, true, true, true>;
+constexpr int kResShapes = 4, kResMaxWords = 2048;
+constexpr int kResClusterBlocks = 16;  // of a cluster at most
 // Host view of a shape: voxel pairs and threads, floats per component, face words per thread.
 struct ResCaps {
   int np, nt, cu, cq, ne;
+  bool cluster;
 };
-template <typename C> constexpr ResCaps res_caps() { return {C::NP, C::NT, C::CU, C::CQ, C::NE}; }
-constexpr ResCaps kResCaps[kResShapes] = {res_caps<ResSmall>(), res_caps<ResMid>(), res_caps<ResLarge<__half>>()};
+template <typename C> constexpr ResCaps res_caps() { return {C::NP, C::NT, C::CU, C::CQ, C::NE, C::CLUSTER}; }
+constexpr ResCaps kResCaps[kResShapes] = {res_caps<ResSmall>(), res_caps<ResMid>(), res_caps<ResLarge<__half>>(),
+                                           res_caps<ResCluster>()};
 
-// op 0: set the kernel's shared-memory attribute and return the CTAs one SM holds in *occ (false:
-// not usable); op 1: one cooperative launch of `grid` CTAs of `threads` threads on stream s.
+// op 0: set the kernel's attributes and return in *occ the CTAs one SM holds, or the clusters of
+// kResClusterBlocks CTAs that the GPU holds (false: not usable); op 1: one launch of `grid` CTAs of `threads`
+// threads on stream s, cooperative or in clusters of L->cluster.
 bool resident_variant(int storage, int shape, int op, unsigned grid, unsigned threads, const ResLaunch* L,
                       const Desc* descs, const ResidentArgs* a, int* status, cudaStream_t s, int* occ);
 

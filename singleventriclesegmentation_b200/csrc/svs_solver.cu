@@ -1031,11 +1031,11 @@ double stream_us(double work, bool groups) {
 // the two exchanges (2.5 us with next to no work), the warps' pairs, the words' traffic, and the
 // launch itself over its iterations. 6x6x6 boxes 2.7 us, 8x8x10 3.4, 10x10x10 4.0 (np 1), 20x8x8
 // 4.6, 40x8x6 5.8, 20x10x10 6.2 (np 2; f32 5.3, 6.4 and 6.8), 20x12x15 9.7, 16x12x20 10.5 (np 5;
-// f32 14.2 and 14.6).
-float resident_us(int storage, int np, int threads, int words, int iters) {
+// f32 13.8). In a cluster the exchanges take 1.5 us: 6x6x6 boxes 1.9 us, 10x10x5 2.3, 12x12x6 3.2, 10x10x10 3.2.
+float resident_us(int storage, int np, int threads, int words, int iters, bool cluster) {
   const bool f32 = storage == SVS_STORAGE_F32;
   const float pair_us = np > 2 ? (f32 ? 0.175f : 0.12f) : np == 2 && f32 ? 0.11f : 0.085f;
-  return 2.45f + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words + 6.0f / iters;
+  return (cluster ? 1.5f : 2.45f) + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words + 6.0f / iters;
 }
 
 // ---- resident iterations (svs_resident.cuh): which pairs of a level, in which boxes
@@ -1056,7 +1056,7 @@ std::vector<ResBoxes> resident_boxes(int storage, int iters, const ResCaps& c) {
         const int col = 2 * bz * by;
         if ((bz + 2) * (by + 2) * bx + col > c.cu || std::max(bz * by * bx + col, std::max(bz * (by + 2) * bx, (bz + 2) * by * bx)) > c.cq)
           continue;
-        out.push_back({bx, by, bz, threads, words, resident_us(storage, c.np, threads, words, iters)});
+        out.push_back({bx, by, bz, threads, words, resident_us(storage, c.np, threads, words, iters, c.cluster)});
       }
   std::sort(out.begin(), out.end(), [](const ResBoxes& a, const ResBoxes& b) { return a.us < b.us; });
   return out;
@@ -1121,6 +1121,9 @@ void plan_resident(svs_plan& P, int level) {
     int occ = 0;
     if (!resident_variant(P.prm.storage, sh, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, &occ)) continue;
     boxes[sh] = resident_boxes(P.prm.storage, P.prm.max_outer_iterations, kResCaps[sh]);
+    // a pair takes boxes of one launch, or one cluster; room for them at once
+    const bool cluster = kResCaps[sh].cluster;
+    const int most = cluster ? kResClusterBlocks : slots, room = cluster ? occ : slots;
     // per pair: fewer boxes for more time
     std::vector<std::vector<Choice>> front(np);
     std::vector<float> bounds;
@@ -1132,7 +1135,7 @@ void plan_resident(svs_plan& P, int level) {
       if (same >= 0) {
         front[i] = front[same];
       } else {
-        int fewest = slots + 1;
+        int fewest = most + 1;
         for (int b = 0; b < (int)boxes[sh].size(); ++b) {
           const int n = resident_count(D[i], boxes[sh][b]);
           if (n <= 0 || n >= fewest) continue;
@@ -1157,12 +1160,13 @@ void plan_resident(svs_plan& P, int level) {
           if (q.us <= bound) c = &q;
         if (!c) { ok = false; break; }
         pick[i] = c->box;
-        if (used + c->count > slots) {
+        const int takes = cluster ? 1 : c->count;
+        if (used + takes > room) {
           total += longest;
           used = 0;
           longest = 0.f;
         }
-        used += c->count;
+        used += takes;
         longest = std::max(longest, c->us);
       }
       total += longest;
@@ -1177,7 +1181,12 @@ void plan_resident(svs_plan& P, int level) {
   }
   if (best_us < 0 || best_us >= streamed(std::vector<int>(np, -1))) return;
   svs_plan::ResStep st;
-  int npairs = 0;
+  int npairs = 0, blocks = 0;  // blocks: of a cluster, a power of two
+  if (kResCaps[best_shape].cluster) {
+    blocks = 1;
+    for (int i = 0; i < np; ++i)
+      while (best_box[i] >= 0 && blocks < resident_count(D[i], boxes[best_shape][best_box[i]])) blocks *= 2;
+  }
   auto flush = [&] {
     if (npairs) P.res_steps[level].push_back(st);
     st = svs_plan::ResStep{};
@@ -1186,8 +1195,8 @@ void plan_resident(svs_plan& P, int level) {
   for (int i = 0; i < np; ++i) {
     if (best_box[i] < 0) continue;
     const ResBoxes& b = boxes[best_shape][best_box[i]];
-    const int n = resident_count(D[i], b);
-    if (st.grid + n > (unsigned)slots) flush();
+    const int n = blocks ? blocks : resident_count(D[i], b);
+    if (st.grid + n > (unsigned)(blocks ? kResSlots : slots)) flush();
     ResPair& r = st.launch.pair[npairs];
     r.desc = level * np + i;
     r.first = (int)st.grid;
@@ -1199,6 +1208,7 @@ void plan_resident(svs_plan& P, int level) {
     r.bz = (unsigned char)b.bz;
     for (int k = 0; k < n; ++k) st.launch.of[st.grid + k] = (unsigned char)npairs;
     st.shape = best_shape;
+    st.launch.cluster = blocks;
     st.grid += (unsigned)n;
     st.threads = std::max(st.threads, (unsigned)ceil_div(b.threads, 32) * 32);
     st.words = std::max(st.words, b.words);

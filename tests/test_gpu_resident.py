@@ -118,3 +118,16 @@ def test_two_streams(cuda):
         solvers[k].plan_for([shape]).check()
         for u in got[k]:
             assert torch.equal(u, want[k])
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16-flow32", "bf16"])
+@pytest.mark.parametrize("shapes,iters", [
+    ([(4, 4, 4)], 3),                                 # one box
+    ([(9, 11, 12)], 7),                               # fewer boxes than a power of two
+    ([(20, 20, 20)], 6),
+    ([(5, 23, 19)], 5),                               # odd sizes
+    ([(10, 11, 9 + i % 4) for i in range(23)], 5),    # more clusters than one launch or the GPU holds
+])
+def test_volumes_in_one_cluster(cuda, storage, shapes, iters):
+    _, plan = both(storage, shapes, 1, 2, iters)
+    assert plan.level_resident(0) == len(shapes)
