@@ -26,16 +26,18 @@
 // word, which ends its neighbours' waits and the plan's later launches.
 //
 // CLUSTER: a volume of at most 16 boxes runs in one thread-block cluster instead. The faces are then
-// written straight into the halo cells of the neighbours' shared memory, and one cluster barrier
-// per exchange replaces words, tags and polling (every box has read its halo before it sends what
-// lets a neighbour write again: the same order as above). No box of another pair is waited for, so the
-// launch is not cooperative. An exchange takes about 0.75 us instead of 1.25: 20^3 2.8 -> 2.3 us per iteration (16 boxes
-// of 10x10x5), 9x11x12 2.7 -> 1.8. From about 250 voxel pairs per box on, the boxes' arithmetic is worth more
-// than that (24^3: 3.2 us in one cluster, 2.7 us on 144 SMs), and the choice below sees it.
+// stored asynchronously into the halo cells of the neighbours' shared memory and counted by an
+// mbarrier there, one per field, which replaces words, tags and polling through L2 (every box has read
+// its halo before it sends what lets a neighbour write again: the same order as above). No box of
+// another pair is waited for, so the launch is not cooperative. An exchange takes about 0.55 us instead of 1.25
+// (0.75 with a cluster barrier per exchange, whose release waits until the stores have arrived):
+// 20^3 2.8 -> 2.0 us per iteration (16 boxes of 10x10x5), 9x11x12 2.7 -> 1.5, 18x21x24 2.85 -> 2.45. From about
+// 200 voxel pairs per box on, the boxes' arithmetic is worth more than that (24^3: 2.6 us on 144 SMs),
+// and the choice in plan_resident sees it.
 //
 // Measured on one B200 (us per iteration; before: one launch per iteration, march along z):
-//   f16-flow32 80^3 10.6 (20.4), 48^3 3.4 (14.4), 40^3 3.3 (10.3), 20^3 2.3 (8.2);
-//   f32 80^3 13.8 (20.5), 48^3 3.4 (12.3), 20^3 2.3 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
+//   f16-flow32 80^3 10.6 (20.4), 48^3 3.4 (14.4), 40^3 3.3 (10.3), 20^3 2.0 (8.2);
+//   f32 80^3 13.8 (20.5), 48^3 3.4 (12.3), 20^3 1.85 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
 // Small boxes are bound by the two exchanges (about 2.5 us: publish, poll, barriers). 80^3 is
 // bound by the latency of 12 warps of 168 registers (about 8,000 cycles of dual, 5,800 of primal)
 // and by the words' L2 traffic (3.6 MB per exchange each way). Its f32 form keeps p alone (90
@@ -97,7 +99,8 @@ struct ResShape {
   // the register file holds 16,384 registers per scheduler, a quarter of the warps each
   static constexpr int WARPS = (NT + 31) / 32, MAXREG = 16384 / ((WARPS + 3) / 4 * 32) / 8 * 8;
   static constexpr int REGS = MAXREG > 255 ? 255 : MAXREG;
-  static constexpr int SMEM = (3 * CU + 9 * CQ) * 4;
+  static constexpr int BAR = (3 * CU + 9 * CQ) * 4;      // CLUSTER: two mbarriers behind the arrays
+  static constexpr int SMEM = BAR + (CLUSTER ? 16 : 0);
   static_assert(SMEM <= 227 * 1024, "fits one CTA per SM");
   static_assert(CU % 2 == 0 && CQ % 2 == 0, "8-byte aligned components");
   static_assert(CU < 65536 && 7 * CQ < 65536, "cells are 16-bit");
@@ -147,16 +150,34 @@ __device__ __forceinline__ uint4 word_poll(const uint4* p, unsigned on) {
       : "memory");
   return v;
 }
-// Shared memory of another CTA of the cluster, and the cluster's barrier (every thread of the cluster
-// that has not returned; what was written before it can be read after it).
+// Shared memory of another CTA of the cluster...
 __device__ __forceinline__ unsigned peer_address(const void* p, unsigned rank) {
   unsigned r;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void peer_store(unsigned p, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(p), "f"(v) : "memory");
+// ...stored to asynchronously; the bytes are counted by an mbarrier of that CTA
+__device__ __forceinline__ void peer_store(unsigned p, float v, unsigned bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(p), "f"(v), "r"(bar)
+               : "memory");
 }
+__device__ __forceinline__ void bar_init(unsigned bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
+  asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ bool bar_done(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok;
+}
+// Every thread of the cluster that has not returned; what was written before can be read after.
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -355,7 +376,7 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
         if constexpr (C::CLUSTER) {
           const unsigned out = peer[i] + 4 * ((q ? 3 * C::CU : 0) + ((q ? qcell[i] : ucell[i]) & 0xffff));
 #pragma unroll
-          for (int c = 0; c < 3; ++c) peer_store(out + 4 * c * st, v[i][c]);
+          for (int c = 0; c < 3; ++c) peer_store(out + 4 * c * st, v[i][c], peer[i] + C::BAR + (q ? 8 : 0));
         } else {
           word_publish(a.xbuf + word[i] + (q ? S : 0), v[i][0], v[i][1], v[i][2], tag);
         }
@@ -400,6 +421,31 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
           return false;
         }
       }
+    }
+    return true;
+  };
+
+  // CLUSTER: the neighbours' faces of one field have arrived (false: gave up). The phase is armed by
+  // thread 0; bytes that came before that are already counted.
+  const unsigned bars = (unsigned)__cvta_generic_to_shared(sm) + C::BAR;
+  unsigned face_bytes = 0;
+  if constexpr (C::CLUSTER) {
+#pragma unroll
+    for (int i = 0; i < C::NE; ++i) face_bytes += 12 * __syncthreads_count(word[i] >= 0);
+    if (tid == 0) {
+      bar_init(bars);
+      bar_init(bars + 8);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+  }
+  auto arrived = [&](bool q, int it) {
+    const unsigned bar = bars + (q ? 8 : 0);
+    uint64_t t0 = 0;
+    for (unsigned spin = 0; !bar_done(bar, it & 1); ++spin) {
+      if ((spin & 31) != 31) continue;
+      const uint64_t now = global_ns();
+      if (!t0) t0 = now;
+      else if (now - t0 > wait_ns) return false;
     }
     return true;
   };
@@ -471,11 +517,18 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       for (int j = 0; j < NP; ++j)
         if (j < nj) load_R(j);
     }
-    __syncthreads();
-    send(true, (unsigned)it + 1);
     if constexpr (C::CLUSTER) {
-      cluster_barrier();
+      if (__syncthreads_or(bad)) {
+        bad = true;
+        break;
+      }
+      if (tid == 0) bar_expect(bars + 8, face_bytes);
+      send(true, (unsigned)it + 1);
+      __syncthreads();
+      bad = !arrived(true, it);
     } else {
+      __syncthreads();
+      send(true, (unsigned)it + 1);
       bad = !receive(true, (unsigned)it + 1);
       if (__syncthreads_or(bad)) {
         bad = true;
@@ -528,11 +581,18 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       }
     }
     if (it + 1 < a.iters) {
-      __syncthreads();
-      send(false, (unsigned)it + 1);
       if constexpr (C::CLUSTER) {
-        cluster_barrier();
+        if (__syncthreads_or(bad)) {
+          bad = true;
+          break;
+        }
+        if (tid == 0) bar_expect(bars, face_bytes);
+        send(false, (unsigned)it + 1);
+        __syncthreads();
+        bad = !arrived(false, it);
       } else {
+        __syncthreads();
+        send(false, (unsigned)it + 1);
         bad = !receive(false, (unsigned)it + 1);
         if (__syncthreads_or(bad)) {
           bad = true;
@@ -541,8 +601,13 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       }
     }
   }
+  if constexpr (C::CLUSTER) bad = __syncthreads_or(bad);
   if (bad) {
     if (tid == 0) atomicOr(status, SVS_DEV_TIMEOUT);
+    if constexpr (C::CLUSTER) {  // until no other block sends any more, and what it sent has landed
+      cluster_barrier();
+      for (const uint64_t t = global_ns(); global_ns() - t < 20000;) {}
+    }
     return;
   }
 

@@ -18,6 +18,8 @@
 // the new dual field on the tile plus a one-voxel x/y halo (recomputed, so no grid-wide
 // dependency between the two half steps) and the new flow on the plane below. The only
 // per-iteration HBM traffic is read u, p, D, rc, gw and write u, p: 34 values per voxel.
+// Volumes that fit the chip run all iterations of a warp in one launch instead, with u, p, D, rc and gw
+// in registers and shared memory (svs_resident.cuh); plan_resident chooses per level and pair.
 // The whole batched solve is captured once into a CUDA graph.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -1031,11 +1033,13 @@ double stream_us(double work, bool groups) {
 // the two exchanges (2.5 us with next to no work), the warps' pairs, the words' traffic, and the
 // launch itself over its iterations. 6x6x6 boxes 2.7 us, 8x8x10 3.4, 10x10x10 4.0 (np 1), 20x8x8
 // 4.6, 40x8x6 5.8, 20x10x10 6.2 (np 2; f32 5.3, 6.4 and 6.8), 20x12x15 9.7, 16x12x20 10.5 (np 5;
-// f32 13.8). In a cluster the exchanges take 1.5 us: 6x6x6 boxes 1.9 us, 10x10x5 2.3, 12x12x6 3.2, 10x10x10 3.2.
+// f32 13.8). In a cluster the exchanges take about 1.1 us: 9x11x12 in 8 boxes
+// 1.5 us, 20^3 in 16 boxes of 10x10x5 2.0, 18x21x24 in 16 2.45; the model is on the high side there, so that a tie
+// (24^3) goes to one box per SM.
 float resident_us(int storage, int np, int threads, int words, int iters, bool cluster) {
   const bool f32 = storage == SVS_STORAGE_F32;
   const float pair_us = np > 2 ? (f32 ? 0.175f : 0.12f) : np == 2 && f32 ? 0.11f : 0.085f;
-  return (cluster ? 1.5f : 2.45f) + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words + 6.0f / iters;
+  return (cluster ? 1.2f : 2.45f) + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words + 6.0f / iters;
 }
 
 // ---- resident iterations (svs_resident.cuh): which pairs of a level, in which boxes
