@@ -31,13 +31,14 @@
 // its halo before it sends what lets a neighbour write again: the same order as above). No box of
 // another pair is waited for, so the launch is not cooperative. An exchange takes about 0.55 us instead of 1.25
 // (0.75 with a cluster barrier per exchange, whose release waits until the stores have arrived):
-// 20^3 2.8 -> 2.0 us per iteration (16 boxes of 10x10x5), 9x11x12 2.7 -> 1.5, 18x21x24 2.85 -> 2.45. From about
+// 20^3 2.8 -> 2.0 us per iteration (16 boxes of 10x10x5), 9x11x12 2.7 -> 1.5, 18x21x24 2.85 -> 2.45
+// (1.85, 1.35 and 2.2 with EARLY below). From about
 // 200 voxel pairs per box on, the boxes' arithmetic is worth more than that (24^3: 2.6 us on 144 SMs),
 // and the choice in plan_resident sees it.
 //
 // Measured on one B200 (us per iteration; before: one launch per iteration, march along z):
-//   f16-flow32 80^3 10.6 (20.4), 48^3 3.4 (14.4), 40^3 3.3 (10.3), 20^3 2.0 (8.2);
-//   f32 80^3 13.8 (20.5), 48^3 3.4 (12.3), 20^3 1.85 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
+//   f16-flow32 80^3 10.6 (20.4), 48^3 3.3 (14.4), 40^3 3.2 (10.3), 20^3 1.85 (8.2);
+//   f32 80^3 13.8 (20.5), 48^3 3.3 (12.3), 20^3 1.85 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
 // Small boxes are bound by the two exchanges (about 2.5 us: publish, poll, barriers). 80^3 is
 // bound by the latency of 12 warps of 168 registers (about 8,000 cycles of dual, 5,800 of primal)
 // and by the words' L2 traffic (3.6 MB per exchange each way). Its f32 form keeps p alone (90
@@ -91,10 +92,13 @@ struct ResidentArgs {
 // is used, the others before the wait for q's halo. ROLL: the primal keeps q_z of two planes from pair
 // to pair instead of reading each plane twice. Taken where p alone is held (f32 80^3 14.7 -> 13.8 us
 // per iteration); with D held too it takes registers that are not there (f16-flow32 80^3 10.6 -> 10.8).
+// EARLY: the part of the primal that needs no q, the step of the shrinkage, is computed between publishing q's
+// faces and waiting for the neighbours' (35x41x47 f16-flow32 3.43 -> 3.27 us, 40^3 3.37 -> 3.2, 20^3 2.0 -> 1.83). The
+// 5-pair shape is short of registers for it (10.6 -> 11.0, f32 13.8 -> 15.7).
 template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_D_, bool KEEP_R_, bool CLUSTER_ = false>
 struct ResShape {
   static constexpr int NP = NP_, NT = NT_, CU = CU_, CQ = CQ_, NE = NE_;
-  static constexpr bool CLUSTER = CLUSTER_;
+  static constexpr bool CLUSTER = CLUSTER_, EARLY = NP <= 2;
   static constexpr bool KEEP_D = KEEP_D_, KEEP_R = KEEP_R_, ROLL = !KEEP_D;
   // the register file holds 16,384 registers per scheduler, a quarter of the warps each
   static constexpr int WARPS = (NT + 31) / 32, MAXREG = 16384 / ((WARPS + 3) / 4 * 32) / 8 * 8;
@@ -353,6 +357,24 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
   }
 
   const float wtv2 = a.wtv * a.wtv;
+  float2 step_len[C::EARLY ? NP : 1];  // EARLY: of the L1 shrinkage, computed while q's faces travel
+  auto early_steps = [&](float factor) {
+    if constexpr (C::EARLY) {
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+        step_len[j] = make_float2(0.f, 0.f);
+        if (j < nj) {
+          float2 uo[3], g[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            uo[c] = *reinterpret_cast<const float2*>(su + c * C::CU + iu + j * PU);
+            g[c] = H::get(R[j][1 + c]);
+          }
+          step_len[j] = primal_step(uo, factor, H::get(R[j][0]), g);
+        }
+      }
+    }
+  };
 
   auto pair_at = [](const float* p) { return *reinterpret_cast<const float2*>(p); };
   const uint4* const in0 = a.xbuf + (long long)blockIdx.x * 2 * S;
@@ -524,11 +546,13 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       }
       if (tid == 0) bar_expect(bars + 8, face_bytes);
       send(true, (unsigned)it + 1);
+      early_steps(factor);
       __syncthreads();
       bad = !arrived(true, it);
     } else {
       __syncthreads();
       send(true, (unsigned)it + 1);
+      early_steps(factor);
       bad = !receive(true, (unsigned)it + 1);
       if (__syncthreads_or(bad)) {
         bad = true;
@@ -555,7 +579,9 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
           uo[c] = pair_at(su + c * C::CU + iu + j * PU);
           g[c] = H::get(R[j][1 + c]);
         }
-        const float2 t = primal_step(uo, factor, H::get(R[j][0]), g);
+        float2 t;
+        if constexpr (C::EARLY) t = step_len[j];
+        else t = primal_step(uo, factor, H::get(R[j][0]), g);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           const float* qx = sqx + c * C::CQ;
