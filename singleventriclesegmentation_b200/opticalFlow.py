@@ -252,8 +252,12 @@ class WarpingCNN3D:
         self._interp = int(interpolation)
         self._bdry = int(boundary)
 
-    def forward(self, u: torch.Tensor, phi: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
-        """u warped by phi; into `out` where given (contiguous, of u's shape, type and device)."""
+    def forward(self, u: torch.Tensor, phi: torch.Tensor) -> torch.Tensor:
+        return self._forward_into(u, phi, None)
+
+    def _forward_into(self, u, phi, out):
+        """u warped by phi into `out`, which no other tensor may share memory with (the kernel gathers
+        from u while it writes); a new tensor for None."""
         _check_input(u, "u")
         _check_input(phi, "phi")
         _check_dim(u, 5)
@@ -264,6 +268,11 @@ class WarpingCNN3D:
         _same_device(u, phi)
         if out is None:
             out = torch.empty_like(u)
+        else:
+            _check_input(out, "out")
+            _same_device(u, out)
+            if out.shape != u.shape:
+                raise RuntimeError("out must have u's shape")
         hz, hy, hx = self._mesh.h()
         call("svs_warp_cnn3d", u, ptr(u), B, C, nz, ny, nx, ptr(phi), hz, hy, hx, self._interp, self._bdry, ptr(out))
         return out

@@ -88,7 +88,7 @@ def propagate_batched(warp: Warp, masks: torch.Tensor, flows: torch.Tensor) -> t
         out = masks.new_empty((flows.shape[0] + 1,) + tuple(masks.shape))
         out[0].copy_(masks)
         for t in range(flows.shape[0]):
-            op.forward(out[t], flows[t].contiguous(), out[t + 1])
+            op._forward_into(out[t], flows[t].contiguous(), out[t + 1])
         return out
     out = [masks]
     for t in range(flows.shape[0]):

@@ -38,6 +38,14 @@ def test_operators_reject_cpu_and_strided_tensors():
         opticalFlow.TVL1OF3D_proxDual(torch.zeros(4, 4, 4, 3, 3), 0.5, 0.025, m)
 
 
+def test_operators_take_no_output_buffers():
+    """The drop-in operators check every tensor they are given and allocate their results."""
+    import inspect
+    for op, inputs in ((opticalFlow.Warping3D, ["u", "phi"]), (opticalFlow.WarpingCNN3D, ["u", "phi"]),
+                       (opticalFlow.Prolongation3D, ["u"])):
+        assert list(inspect.signature(op.forward).parameters) == ["self"] + inputs
+
+
 def test_blur_kernel_is_the_reference_kernel():
     k = gaussian_kernel3d(1.0)
     assert tuple(k.shape) == (5, 5, 5)
