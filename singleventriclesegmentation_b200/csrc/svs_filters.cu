@@ -161,7 +161,7 @@ median3_kernel(const T* __restrict__ in, int nz, int ny, int nx, int C, T* __res
   }
 }
 
-// Generic odd window (7, and 5 of doubles): partial selection sort in local memory up to the median rank.
+// Generic odd window (7, and 5 of doubles or of rows beyond 2^31 elements): partial selection sort in local memory up to the median rank.
 template <typename T>
 __global__ void median_generic_kernel(const T* __restrict__ in, int nz, int ny, int nx, int C,
                                       int ks, T* __restrict__ out) {
@@ -269,6 +269,12 @@ median5_kernel(const float* __restrict__ in, int nz, int ny, int nx, int C, floa
   }
 }
 
+// median5_kernel indexes a row (nx voxels of C components) with 32 bits; longer rows take the general kernel.
+constexpr bool median5_row_fits(int nx, int C) { return (int64_t)nx * C <= INT_MAX; }
+static_assert(median5_row_fits(80, 3) && median5_row_fits(INT_MAX, 1) && !median5_row_fits(1 << 30, 2) &&
+                  !median5_row_fits(50000, 50000),
+              "no row of more than 2^31 - 1 elements");
+
 unsigned grid_for(int64_t n, int threads) {
   const int64_t blocks = (n + threads - 1) / threads;
   return (unsigned)(blocks < 148 * 64 ? (blocks > 0 ? blocks : 1) : 148 * 64);
@@ -310,7 +316,7 @@ svs_status median3d(const char* nm, const T* in, int nz, int ny, int nx, int C, 
     return check_launch(nm);
   }
   if constexpr (sizeof(T) == 4)
-    if (ks == 5) {
+    if (ks == 5 && median5_row_fits(nx, C)) {
       median5_kernel<<<grid_for(n, 128), 128, 0, stream>>>(in, nz, ny, nx, C, out);
       return check_launch(nm);
     }
