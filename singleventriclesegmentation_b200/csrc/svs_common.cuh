@@ -31,7 +31,8 @@ inline unsigned ceil_div(int64_t a, int64_t b) { return (unsigned)((a + b - 1) /
 // Index folding of boundary.cuh:25-46 (a single fold), followed by a clamp so that no sample is
 // ever read outside the array: the reference reads out of bounds when a sample lies more than
 // one volume length outside (boundary.cuh:33-46). The fold is a switch, not the reference's
-// device function-pointer table (boundary.cuh:54), so it inlines.
+// device function-pointer table (boundary.cuh:54), so it inlines. The arithmetic on i must not
+// overflow (safe_index): the compiler orders clamps and additions on the strength of that.
 __device__ __forceinline__ int fold(int i, int n, int bdry) {
   int f = i;
   if (bdry != SVS_BOUNDARY_NEAREST) {  // MIRROR repeats the face's node, REFLECT does not
@@ -44,15 +45,20 @@ __device__ __forceinline__ int fold(int i, int n, int bdry) {
 // The helpers below are templates on the value type T (float, or double for the FP64 forms of
 // the per-operator entry points); the float instantiations are the arithmetic of the reference's
 // float path.
-__device__ __forceinline__ float tfloor(float v) { return floorf(v); }
-__device__ __forceinline__ double tfloor(double v) { return floor(v); }
+// Floor of a grid coordinate as a 32-bit index: saturated beyond the range (defined for every
+// value, unlike a cast), and kept far enough inside it that a tap's offset and its fold cannot overflow.
+// With a saturated index, index + 2 overflowed, and the compiler, which may move an addition out of the
+// clamp to the volume, read out of range. Indices that far out fold to a face either way.
+__device__ __forceinline__ int floor_index(float g) { return __float2int_rd(g); }
+__device__ __forceinline__ int floor_index(double g) { return __double2int_rd(g); }
+__device__ __forceinline__ int safe_index(int i) { return min(max(i, -0x7fffff00), 0x7fffff00); }
 
 // 1D Catmull-Rom through 4 samples in the reference's coefficient form
 // (interpolation_cubicHermiteSpline.cuh:20-56), evaluated at buffer coordinate w + 1.
 template <typename T>
 __device__ __forceinline__ T hermite4(T b0, T b1, T b2, T b3, T w) {
   const T local = w + T(1);
-  const int kf = (int)tfloor(local);
+  const int kf = floor_index(local);
   T out;
   if (kf == 1) {
     const T pf = b1, dpf = (b2 - b0) / 2, pc = b2, dpc = (b3 - b1) / 2;
@@ -87,8 +93,9 @@ using FieldRef = FieldRefT<float>;
 template <typename T>
 __device__ __forceinline__ void split_coord(T c, T h, int& i, T& w) {
   const T g = h == T(1) ? c : c / h;
-  i = (int)tfloor(g);
-  w = g - (T)i;
+  const int k = floor_index(g);
+  w = g - (T)k;
+  i = safe_index(k);
 }
 
 // Tricubic sample (interpolation_cubicHermiteSpline.cuh:482-525, and the vector/matrix/CNN
@@ -241,8 +248,8 @@ __device__ __forceinline__ T sample_linear(const FieldRefT<T>& f, T cz, T cy, T 
 template <typename T>
 __device__ __forceinline__ int nearest_axis(T c, T h, int n, int bdry) {
   const T g = c / h;
-  const int f = (int)tfloor(g);
-  const T df = g - (T)f;
+  const int k = floor_index(g), f = safe_index(k);
+  const T df = g - (T)k;
   const T dc = (T)(f + 1) - g;
   return fold(df < dc ? f : f + 1, n, bdry);
 }
