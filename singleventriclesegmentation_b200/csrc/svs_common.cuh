@@ -166,8 +166,9 @@ __device__ __forceinline__ Two<T> hermite_two(Two<T> b0, Two<T> b1, Two<T> b2, T
 }
 
 // Where one tricubic sample lies, found once for all fields sampled there: its window's first tap
-// and the position in the window per axis. `plain` is false where w + 1 rounds up to 2 on some axis:
-// hermite4's shifted window, left to sample_cubic.
+// and the position in the window per axis. `plain` says that every axis takes hermite4's first branch,
+// 1 <= w + 1 < 2. The others are left to sample_cubic: w + 1 rounded up to 2 (the shifted window), and
+// coordinates beyond the 32-bit range, whose saturated index leaves w at any distance, or NaN.
 template <typename T>
 struct CubicTaps {
   int x, y, z;
@@ -182,11 +183,11 @@ __device__ __forceinline__ CubicTaps<T> cubic_taps(T cz, T cy, T cx, T hz, T hy,
   split_coord(cy, hy, k.y, wy);
   split_coord(cz, hz, k.z, wz);
   const T lx = wx + T(1), ly = wy + T(1), lz = wz + T(1);
-  --k.x, --k.y, --k.z;
   k.tx = lx - T(1);
   k.ty = ly - T(1);
   k.tz = lz - T(1);
-  k.plain = lx < T(2) && ly < T(2) && lz < T(2);
+  k.plain = lx >= T(1) && lx < T(2) && ly >= T(1) && ly < T(2) && lz >= T(1) && lz < T(2);
+  if (k.plain) --k.x, --k.y, --k.z;
   return k;
 }
 // The sample of one field of fewer than 2^31 elements (x step sx). The four planes one after the

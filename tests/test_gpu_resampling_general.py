@@ -29,7 +29,7 @@ def far_flow(ny, nx, axis, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-@pytest.mark.parametrize("interp", ["NEAREST", "LINEAR"])
+@pytest.mark.parametrize("interp", ["NEAREST", "LINEAR", "CUBIC_HERMITESPLINE"])
 @pytest.mark.parametrize("boundary", ["NEAREST", "MIRROR", "REFLECT"])
 @pytest.mark.parametrize("axis", [0, 1, 2])
 def test_far_samples_equal_the_general_kernel(cuda, dtype, interp, boundary, axis):
