@@ -332,6 +332,14 @@ int64_t svs_tvl1_plan_level_ctas(const svs_plan* plan, int level);
  * boundary, unit spacing, no variant, chunk, persistent or stall request at the level); results
  * are bitwise those of the split-role variants. */
 int svs_tvl1_plan_level_resident(const svs_plan* plan, int level);
+/* The compiled shape these pairs run in (after the first solve): 0 none; 1, 2, 3: one, two or five
+ * voxel pairs per thread, one box per SM; 4: one pair per thread, a volume in one thread-block cluster. */
+int svs_tvl1_plan_level_resident_shape(const svs_plan* plan, int level);
+/* Whether the plan may keep iterations on chip (the default). Off: one launch per iteration at
+ * every level, as with an explicit variant but with the automatic variants; bitwise the same flows.
+ * For programs whose many small solves overlap on several streams (on-chip solves of more than
+ * one thread-block cluster take turns), and for timing the per-iteration kernels. */
+svs_status svs_tvl1_plan_set_resident(svs_plan* plan, int on);
 /* The z-chunk plan of the split-role kernels (host arithmetic only, no device needed): for
  * `columns` column tiles of up to `nz` planes on `slots` resident CTAs (SMs x CTAs per SM), the
  * first columns - tail_columns march in main_chunks chunks each and the last tail_columns in

@@ -613,6 +613,7 @@ struct svs_plan {
   };
   std::vector<std::vector<ResStep>> res_steps;  // [level]
   std::vector<std::vector<char>> resident;      // [level][pair]
+  bool want_resident = true;               // svs_tvl1_plan_set_resident
   bool no_resident = false;                // the launches could not be captured here
   uint4* d_xbuf = nullptr;                 // exchange words, then the abort word
   size_t xbuf_bytes = 0;
@@ -1089,7 +1090,7 @@ void plan_resident(svs_plan& P, int level) {
                    (level < (int)P.level_chunks_req.size() && P.level_chunks_req[level] > 0) ||
                    (level < (int)P.pair_tile_req.size() &&
                     std::any_of(P.pair_tile_req[level].begin(), P.pair_tile_req[level].end(), [](int t) { return t > 0; }));
-  if (req || P.persistent || P.no_resident || P.stall_level == level || P.prm.max_outer_iterations < 2) return;
+  if (req || !P.want_resident || P.persistent || P.no_resident || P.stall_level == level || P.prm.max_outer_iterations < 2) return;
   int dev = 0, sms = 148, coop = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2058,6 +2059,18 @@ int64_t svs_tvl1_plan_level_ctas(const svs_plan* P, int level) {
 int svs_tvl1_plan_level_resident(const svs_plan* P, int level) {
   if (!P || level < 0 || level >= (int)P->resident.size()) return 0;
   return (int)std::count(P->resident[level].begin(), P->resident[level].end(), (char)1);
+}
+
+int svs_tvl1_plan_level_resident_shape(const svs_plan* P, int level) {
+  if (!P || level < 0 || level >= (int)P->res_steps.size() || P->res_steps[level].empty()) return 0;
+  return P->res_steps[level][0].shape + 1;
+}
+
+svs_status svs_tvl1_plan_set_resident(svs_plan* P, int on) {
+  SVS_REQUIRE(P, "svs_tvl1_plan_set_resident: null plan");
+  P->want_resident = on != 0;
+  ++P->tile_epoch;  // rebuild the per-level choice and recapture the graph
+  return SVS_OK;
 }
 
 svs_status svs_tvl1_plan_check(svs_plan* P) {

@@ -126,6 +126,14 @@ class SolverPlan:
         """Pairs of `level` whose iterations run on chip, all of a warp in one launch (after a solve)."""
         return int(_lib.lib().svs_tvl1_plan_level_resident(self._h, int(level)))
 
+    def level_resident_shape(self, level: int) -> int:
+        """Compiled shape of these pairs (svs_tvl1_plan_level_resident_shape; 0 = none on chip)."""
+        return int(_lib.lib().svs_tvl1_plan_level_resident_shape(self._h, int(level)))
+
+    def set_resident(self, on: bool = True) -> None:
+        """Whether iterations may stay on chip (the default); off: one launch per iteration."""
+        check(_lib.lib().svs_tvl1_plan_set_resident(self._h, int(bool(on))))
+
     def level_ctas(self, level: int) -> int:
         """CTAs of one per-iteration launch at `level` (all variant groups; 0 before the first solve)."""
         return int(_lib.lib().svs_tvl1_plan_level_ctas(self._h, int(level)))
