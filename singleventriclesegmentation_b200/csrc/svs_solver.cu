@@ -567,7 +567,12 @@ struct svs_plan {
   bool want_p = false;
   bool warm = false;
   cudaStream_t cap_stream = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  // the captured solve in launch order: up to the first launch whose CTAs wait for one another across
+  // clusters, from there to the last such launch (ResidentTurn), and the rest; without such launches
+  // all of it is the first part
+  cudaGraphExec_t exec[3] = {};
+  cudaGraph_t part[3] = {};                // while capturing
+  int parts = 0;
   uint64_t graph_kernels = 0;
   int graph_tile = -1;
   bool graph_warm = false;
@@ -964,46 +969,52 @@ void build_tiles(svs_plan& P, int level, int tid, std::vector<Tile>* out_opt = n
   out.insert(out.end(), tail.begin(), tail.end());
 }
 
-// Work that holds resident launches takes turns on a device: their CTAs wait for one another, so
-// two such launches from two streams must not each hold a part of the SMs. (A cooperative launch
-// starts only as a whole; this does not lean on two of them never interleaving.) The constructor
-// makes the stream wait for the previous turn, the destructor ends this one. A stream under
-// capture takes none: events cannot cross into a capture.
+// Launches whose CTAs wait for one another (cooperative ones) take turns on a device: two of them from
+// two streams must not each hold a part of the SMs. (A cooperative launch starts only as a whole; this
+// does not lean on two of them never interleaving.) The constructor makes the stream wait for the
+// previous turn, the destructor ends this one. A stream under capture takes none: events cannot cross
+// into a capture. A turn covers a solve from its first such launch to its last, not its other levels:
+// a volume in one cluster waits for no other, and per-iteration launches of several streams fill the GPU
+// together. (One solve on each of 8 streams, 3 levels x 5 warps x 100 iterations: 18^3 2.8 ms, 32^3 9.9, 96^3
+// 127; with whole solves in turns 21.0, 22.1 and 150; per-iteration launches alone 11.1, 18.6 and 143.)
 class ResidentTurn {
  public:
   explicit ResidentTurn(cudaStream_t s, bool on = true) : s_(s) {
     cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-    if (!on || cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= kDevices ||
+    int dev = 0;
+    if (!on || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices ||
         cudaStreamIsCapturing(s, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone)
       return;
-    lock_ = std::unique_lock<std::mutex>(mutex());
-    cudaEvent_t& e = event(dev_);
-    if (e && cudaStreamWaitEvent(s, e, 0) != cudaSuccess) {  // the device was reset
+    t_ = &turns()[dev];
+    t_->mutex.lock();
+    if (t_->last && cudaStreamWaitEvent(s, t_->last, 0) != cudaSuccess) {  // the device was reset
       cudaGetLastError();
-      e = nullptr;
+      t_->last = nullptr;
     }
-    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+    if (!t_->last && cudaEventCreateWithFlags(&t_->last, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
-      e = nullptr;
+      t_->last = nullptr;
     }
   }
   ~ResidentTurn() {
-    if (lock_.owns_lock() && event(dev_)) cudaEventRecord(event(dev_), s_);
+    if (!t_) return;
+    if (t_->last) cudaEventRecord(t_->last, s_);
+    t_->mutex.unlock();
   }
+  ResidentTurn(const ResidentTurn&) = delete;
 
  private:
   static constexpr int kDevices = 64;
-  static std::mutex& mutex() {
-    static std::mutex m;
-    return m;
-  }
-  static cudaEvent_t& event(int dev) {
-    static cudaEvent_t e[kDevices] = {};
-    return e[dev];
+  struct Turns {
+    std::mutex mutex;
+    cudaEvent_t last = nullptr;
+  };
+  static Turns* turns() {
+    static Turns t[kDevices];
+    return t;
   }
   cudaStream_t s_;
-  int dev_ = 0;
-  std::unique_lock<std::mutex> lock_;
+  Turns* t_ = nullptr;
 };
 
 // Modelled microseconds per iteration, fitted to measurements on one B200.
@@ -1233,6 +1244,15 @@ bool all_resident(const svs_plan& P, int level) {
          std::all_of(P.resident[level].begin(), P.resident[level].end(), [](char c) { return c != 0; });
 }
 
+// Whether a level's launches wait across clusters (ResidentTurn).
+bool takes_turn(const svs_plan& P, int level) {
+  if (P.prm.max_outer_iterations < 1 || P.prm.max_warps < 1) return false;
+  if (level < (int)P.level_persist.size() && P.level_persist[level]) return true;
+  for (const svs_plan::ResStep& st : P.res_steps[level])
+    if (!kResCaps[st.shape].cluster) return true;
+  return false;
+}
+
 // `iters` iterations of the level's resident pairs, from ping-pong copy `cur` to cur ^ (iters & 1).
 // Returns the launches issued, -1 after a launch error.
 int resident_iterations(svs_plan& P, int level, int iters, int cur, cudaStream_t s) {
@@ -1455,7 +1475,14 @@ int level_iteration(svs_plan& P, int l, const IterArgs& a_in, cudaStream_t s) {
   return 1 + (int)level_groups(P, l);
 }
 
-// The whole batched solve as a sequence of launches on stream s. Returns the number of kernel
+// During capture on s: what follows belongs to part `k` of the solve.
+bool start_part(svs_plan& P, int k, cudaStream_t s) {
+  if (cudaStreamEndCapture(s, &P.part[P.parts]) != cudaSuccess) return false;
+  P.parts = k;
+  return cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+}
+
+// The whole batched solve as a sequence of launches on stream s (under capture). Returns the number of kernel
 // launches issued or -1 after a launch error.
 template <typename SU, typename SP>
 long long enqueue_solve(svs_plan& P, cudaStream_t s) {
@@ -1478,6 +1505,12 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
     ++launches;
   }
   int cur = 0;
+  int first_turn = -1, last_turn = L;  // levels, coarse to fine
+  for (int l = 0; l < L; ++l)
+    if (takes_turn(P, l)) {
+      first_turn = l;
+      last_turn = std::min(last_turn, l);
+    }
   for (int l = L - 1; l >= 0; --l) {
     const int zero = (l == L - 1) && !(P.warm && L == 1);
     prepare_kernel<SU, SP><<<grid(l), 256, 0, s>>>(D + (size_t)l * np, q.use_anisotropic_diff, q.alpha, q.beta, q.boundary, zero, cur);
@@ -1487,6 +1520,7 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
       residual_kernel<SU><<<grid(l), 256, 0, s>>>(D + (size_t)l * np, cur, P.d_snaps, P.d_acc, 1);
       launches += 2;
     }
+    if (l == first_turn && !start_part(P, 1, s)) return -1;
     for (int w = 0; w < q.max_warps; ++w) {
       linearise_kernel<SU, SP><<<grid(l), 256, 0, s>>>(D + (size_t)l * np, cur, q.interpolation, q.boundary);
       ++launches;
@@ -1520,13 +1554,13 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
         if (all_resident(P, l)) {
           cur ^= q.max_outer_iterations & 1;
         } else {
-        fork_groups(P, l, s);
-        for (int it = 0; it < q.max_outer_iterations; ++it) {
-          const IterArgs a = iter_args(P, it, cur);
-          launches += level_iteration(P, l, a, s);
-          cur ^= 1;
-        }
-        join_groups(P, l, s);
+          fork_groups(P, l, s);
+          for (int it = 0; it < q.max_outer_iterations; ++it) {
+            const IterArgs a = iter_args(P, it, cur);
+            launches += level_iteration(P, l, a, s);
+            cur ^= 1;
+          }
+          join_groups(P, l, s);
         }
       }
       if (P.res_on) {
@@ -1536,6 +1570,7 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
         launches += 2;
       }
     }
+    if (first_turn >= 0 && l == last_turn && !start_part(P, 2, s)) return -1;
     if (l > 0) {
       if (q.interpolation == SVS_INTERPOLATE_CUBIC_HERMITESPLINE && coarse_within(P, l))
         prolong_cubic_kernel<SU, SP><<<dim3(prolong_blocks(P, l - 1), np), PFX * PFY, 0, s>>>(
@@ -1568,6 +1603,27 @@ long long enqueue(svs_plan& P, cudaStream_t s) {
     case SVS_STORAGE_BF16_FLOW32: return enqueue_solve<float, __nv_bfloat16>(P, s);
     case SVS_STORAGE_F16_FLOW32: return enqueue_solve<float, __half>(P, s);
     default: return enqueue_solve<float, float>(P, s);
+  }
+}
+
+// Captures the solve on P.cap_stream into P.part; returns the launches, -1 after an error.
+long long capture_solve(svs_plan& P) {
+  P.parts = 0;
+  if (cudaStreamBeginCapture(P.cap_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return -1;
+  const long long n = enqueue(P, P.cap_stream);
+  if (cudaStreamEndCapture(P.cap_stream, &P.part[P.parts]) != cudaSuccess) return -1;
+  return n;
+}
+void drop_parts(svs_plan& P) {
+  for (cudaGraph_t& g : P.part) {
+    if (g) cudaGraphDestroy(g);
+    g = nullptr;
+  }
+}
+void drop_exec(svs_plan& P) {
+  for (cudaGraphExec_t& e : P.exec) {
+    if (e) cudaGraphExecDestroy(e);
+    e = nullptr;
   }
 }
 
@@ -1788,7 +1844,7 @@ svs_status svs_tvl1_plan_create(const svs_tvl1_params* prm, int num_pairs, const
 
 svs_status svs_tvl1_plan_destroy(svs_plan* P) {
   if (!P) return SVS_OK;
-  if (P->exec) cudaGraphExecDestroy(P->exec);
+  drop_exec(*P);
   if (P->cap_stream) cudaStreamDestroy(P->cap_stream);
   for (auto* t : P->d_tiles) cudaFree(t);
   cudaFree(P->d_descs); cudaFree(P->d_raw); cudaFree(P->d_uout); cudaFree(P->d_umed);
@@ -1934,42 +1990,40 @@ svs_status svs_tvl1_solve_batch(svs_plan* P, const svs_pair_desc* pairs, int num
     if (st) return st;
     P->tiles_built_for = P->tile_epoch;
   }
-  if (!P->exec || P->graph_tile != P->tile_epoch || P->graph_warm != warm || P->graph_want_p != want_p) {
-    if (P->exec) { cudaGraphExecDestroy(P->exec); P->exec = nullptr; }
-    cudaGraph_t g = nullptr;
-    st = check_cuda(cudaStreamBeginCapture(P->cap_stream, cudaStreamCaptureModeThreadLocal), "solve: capture");
-    if (st) return st;
-    long long nl = enqueue(*P, P->cap_stream);
-    cudaError_t ce = cudaStreamEndCapture(P->cap_stream, &g);
-    if ((nl < 0 || ce != cudaSuccess) && (P->persistent || any_resident(*P))) {
+  if (!P->exec[0] || P->graph_tile != P->tile_epoch || P->graph_warm != warm || P->graph_want_p != want_p) {
+    drop_exec(*P);
+    long long nl = capture_solve(*P);
+    if (nl < 0 && (P->persistent || any_resident(*P))) {
       // the cooperative launches of the persistent loop or the resident iterations could not be
       // captured here: per-iteration launches instead (svs_tvl1_plan_level_persistent reports 0)
-      if (g) cudaGraphDestroy(g);
-      g = nullptr;
+      drop_parts(*P);
       cudaGetLastError();
       P->persistent = false;
       P->no_resident = true;
       st = setup_tiles(*P);
       if (st) return st;
-      st = check_cuda(cudaStreamBeginCapture(P->cap_stream, cudaStreamCaptureModeThreadLocal), "solve: capture");
-      if (st) return st;
-      nl = enqueue(*P, P->cap_stream);
-      ce = cudaStreamEndCapture(P->cap_stream, &g);
+      nl = capture_solve(*P);
     }
-    if (nl < 0) { if (g) cudaGraphDestroy(g); return fail(SVS_ERR_LAUNCH, std::string("solve: launch failed during capture: ") + cudaGetErrorString(cudaGetLastError())); }
-    st = check_cuda(ce, "solve: end capture");
-    if (st) return st;
-    st = check_cuda(cudaGraphInstantiate(&P->exec, g, 0), "solve: graph instantiate");
-    cudaGraphDestroy(g);
-    if (st) return st;
+    if (nl < 0) {
+      drop_parts(*P);
+      return fail(SVS_ERR_LAUNCH, std::string("solve: launch failed during capture: ") + cudaGetErrorString(cudaGetLastError()));
+    }
+    for (int k = 0; k < 3 && !st; ++k)
+      if (P->part[k]) st = check_cuda(cudaGraphInstantiate(&P->exec[k], P->part[k], 0), "solve: graph instantiate");
+    drop_parts(*P);
+    if (st) {
+      drop_exec(*P);
+      return st;
+    }
     P->graph_kernels = (uint64_t)nl;
     P->graph_tile = P->tile_epoch;
     P->graph_warm = warm;
     P->graph_want_p = want_p;
   }
-  {
-    ResidentTurn turn(any_resident(*P) ? s : nullptr, any_resident(*P));
-    st = check_cuda(cudaGraphLaunch(P->exec, s), "solve: graph launch");
+  for (int k = 0; k < 3 && !st; ++k) {
+    if (!P->exec[k]) continue;
+    ResidentTurn turn(s, k == 1);
+    st = check_cuda(cudaGraphLaunch(P->exec[k], s), "solve: graph launch");
   }
   if (st) return st;
   count_launches(P->graph_kernels);
@@ -1994,7 +2048,7 @@ svs_status svs_tvl1_bench_iterations(svs_plan* P, int level, int count, svs_stre
   int cur = 0;
   uint64_t launches = 0;
   if (!P->res_steps[level].empty()) {
-    ResidentTurn turn(stream);
+    ResidentTurn turn(stream, takes_turn(*P, level));
     cudaMemsetAsync(P->d_xbuf, 0, P->xbuf_bytes, stream);
     for (int done = 0; done < count; done += P->prm.max_outer_iterations) {
       const int n = std::min(count - done, P->prm.max_outer_iterations);

@@ -7,8 +7,9 @@ HBM budget, and queues the 2(T-1) frame pairs of every admitted request. A batch
 the head of that queue, from as many requests as fit, up to a voxel target that fills the GPU,
 and runs as one batched solve on one of two plans that are re-targeted to each batch without
 allocating (svs_tvl1_plan_retarget): while one batch runs, the next is formed and launched on the
-other plan, so pairs of requests that arrived while others were on the GPU join the next batch
-and their work overlaps on the device. When the last pair of a request is done, its masks are
+other plan, so pairs of requests that arrived while others were on the GPU join the next batch.
+The two plans' levels with one launch per iteration share the GPU; levels whose iterations stay on
+chip take turns (each fills the GPU). When the last pair of a request is done, its masks are
 propagated on the device and its flows and masks are copied to pinned host memory; its latency
 runs from submit() to that copy being complete. Pyramids, dual state and the captured solve
 graphs stay on the device in the plans.
