@@ -26,8 +26,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -1048,23 +1050,30 @@ double stream_us(double work, bool groups) {
 // f32 13.8). In a cluster the exchanges take about 1.1 us: 9x11x12 in 8 boxes
 // 1.5 us, 20^3 in 16 boxes of 10x10x5 2.0, 18x21x24 in 16 2.45; the model is on the high side there, so that a tie
 // (24^3) goes to one box per SM.
-float resident_us(int storage, int np, int threads, int words, int iters, bool cluster) {
+constexpr int kResMaxBx = 64, kResMaxByz = 48;  // of a box
+double launch_us(int iters) { return 6.0 / iters; }
+float resident_us(int storage, int np, int threads, int words, bool cluster) {
   const bool f32 = storage == SVS_STORAGE_F32;
   const float pair_us = np > 2 ? (f32 ? 0.175f : 0.12f) : np == 2 && f32 ? 0.11f : 0.085f;
-  return (cluster ? 1.2f : 2.45f) + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words + 6.0f / iters;
+  return (cluster ? 1.2f : 2.45f) + pair_us * (float)(ceil_div(threads, 32) * np) + 0.0006f * words;
 }
 
 // ---- resident iterations (svs_resident.cuh): which pairs of a level, in which boxes
 struct ResBoxes {
-  int bx, by, bz, threads, words;
-  float us;  // modelled time per iteration
+  unsigned char bx, by, bz;
+  short threads, words;
+  int next;  // first box of another (x, y) extent
+  float us;  // modelled time per iteration, less the launch's part
 };
-// Boxes that fit a compiled shape, by modelled time: x in pairs, z in whole groups of NP pairs.
-std::vector<ResBoxes> resident_boxes(int storage, int iters, const ResCaps& c) {
+// Boxes that fit a compiled shape: x in pairs, z in whole groups of NP pairs (z fastest), the widest
+// first: of boxes that are modelled alike the first is taken, and of the same box in several orientations
+// the wide one is the faster (40^3 10x8x6 2.90 us per iteration, 8x6x10 2.98; 20^3 in a cluster 10x10x5
+// 1.80, 10x5x10 1.91; 12 x 40^3 f32 40x8x6 18.8, 6x8x40 22.6; the exception seen: 32^3 8x8x4 2.10, 4x8x8 2.04).
+std::vector<ResBoxes> list_boxes(int storage, const ResCaps& c) {
   std::vector<ResBoxes> out;
-  for (int bx = 4; bx <= 64; bx += 2)
-    for (int by = 2; by <= 48; ++by)
-      for (int bz = std::max(2, c.np); bz <= 48; bz += c.np) {
+  for (int bx = kResMaxBx; bx >= 4; bx -= 2)
+    for (int by = kResMaxByz; by >= 2; --by)
+      for (int bz = std::max(2, c.np); bz <= kResMaxByz; bz += c.np) {
         const int threads = bx / 2 * by * (bz / c.np);
         const int words = 2 * (bz * by + bz * bx + by * bx);
         if (threads > c.nt) break;
@@ -1072,16 +1081,31 @@ std::vector<ResBoxes> resident_boxes(int storage, int iters, const ResCaps& c) {
         const int col = 2 * bz * by;
         if ((bz + 2) * (by + 2) * bx + col > c.cu || std::max(bz * by * bx + col, std::max(bz * (by + 2) * bx, (bz + 2) * by * bx)) > c.cq)
           continue;
-        out.push_back({bx, by, bz, threads, words, resident_us(storage, c.np, threads, words, iters, c.cluster)});
+        out.push_back({(unsigned char)bx, (unsigned char)by, (unsigned char)bz, (short)threads, (short)words, 0,
+                       resident_us(storage, c.np, threads, words, c.cluster)});
       }
-  std::sort(out.begin(), out.end(), [](const ResBoxes& a, const ResBoxes& b) { return a.us < b.us; });
+  for (int b = (int)out.size() - 1, next = b + 1; b >= 0; --b) {
+    if (b + 1 < (int)out.size() && (out[b].bx != out[b + 1].bx || out[b].by != out[b + 1].by)) next = b + 1;
+    out[b].next = next;
+  }
   return out;
+}
+// ...made once: they depend on nothing but the shape and whether fields have 4 bytes
+const std::vector<ResBoxes>& resident_boxes(int storage, int shape) {
+  static const auto table = [] {
+    std::array<std::array<std::vector<ResBoxes>, kResShapes>, 2> t;
+    for (int wide = 0; wide < 2; ++wide)
+      for (int sh = 0; sh < kResShapes; ++sh)
+        t[wide][sh] = list_boxes(wide ? SVS_STORAGE_F32 : SVS_STORAGE_F16, kResCaps[sh]);
+    return t;
+  }();
+  return table[storage == SVS_STORAGE_F32][shape];
 }
 // Boxes of a volume with no box one voxel thick at its end (the mirrored cell and its source lie
 // in one box), 0 if that fails.
+int axis_count(int n, int b) { return n % b == 1 ? 0 : (n + b - 1) / b; }
 int resident_count(const Desc& d, const ResBoxes& b) {
-  if (d.nx % b.bx == 1 || d.ny % b.by == 1 || d.nz % b.bz == 1) return 0;
-  return (int)(ceil_div(d.nx, b.bx) * ceil_div(d.ny, b.by) * ceil_div(d.nz, b.bz));
+  return axis_count(d.nx, b.bx) * axis_count(d.ny, b.by) * axis_count(d.nz, b.bz);
 }
 // The stencils of resident_kernel: MIRROR, unit spacing, at least 4 nodes per axis.
 bool resident_ok(const svs_plan& P, const Desc& d) {
@@ -1116,7 +1140,18 @@ void plan_resident(svs_plan& P, int level) {
   double best_us = -1.0;
   int best_shape = -1;
   std::vector<int> best_box;
-  std::vector<std::vector<ResBoxes>> boxes(kResShapes);
+  const float launch = (float)launch_us(P.prm.max_outer_iterations);
+  std::vector<int> same(np, -1);  // the first pair of the same size
+  {
+    std::map<std::array<int, 3>, int> seen;
+    for (int i = 0; i < np; ++i) same[i] = seen.emplace(std::array<int, 3>{D[i].nz, D[i].ny, D[i].nx}, i).first->second;
+  }
+  std::vector<std::array<std::array<int, kResMaxBx + 1>, 3>> counts(np);  // boxes along z, y, x by extent
+  for (int i = 0; i < np; ++i) {
+    const int n[3] = {D[i].nz, D[i].ny, D[i].nx};
+    for (int axis = 0; axis < 3 && same[i] == i && resident_ok(P, D[i]); ++axis)
+      for (int b = 2; b <= (axis == 2 ? kResMaxBx : kResMaxByz); ++b) counts[i][axis][b] = axis_count(n[axis], b);
+  }
   std::vector<double> work(np);
   std::vector<int> variant(np);
   for (int i = 0; i < np; ++i) work[i] = stream_pair_us(P.prm.storage, D[i], &variant[i]);
@@ -1136,7 +1171,8 @@ void plan_resident(svs_plan& P, int level) {
   for (int sh = 0; sh < kResShapes; ++sh) {
     int occ = 0;
     if (!resident_variant(P.prm.storage, sh, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, &occ)) continue;
-    boxes[sh] = resident_boxes(P.prm.storage, P.prm.max_outer_iterations, kResCaps[sh]);
+    const std::vector<ResBoxes>& boxes = resident_boxes(P.prm.storage, sh);
+    const long long box_voxels = 2ll * kResCaps[sh].np * kResCaps[sh].nt;
     // a pair takes boxes of one launch, or one cluster; room for them at once
     const bool cluster = kResCaps[sh].cluster;
     const int most = cluster ? kResClusterBlocks : slots, room = cluster ? occ : slots;
@@ -1145,63 +1181,89 @@ void plan_resident(svs_plan& P, int level) {
     std::vector<float> bounds;
     for (int i = 0; i < np; ++i) {
       if (!resident_ok(P, D[i])) continue;
-      int same = -1;
-      for (int k = 0; k < i && same < 0; ++k)
-        if (D[k].nx == D[i].nx && D[k].ny == D[i].ny && D[k].nz == D[i].nz) same = k;
-      if (same >= 0) {
-        front[i] = front[same];
-      } else {
-        int fewest = most + 1;
-        for (int b = 0; b < (int)boxes[sh].size(); ++b) {
-          const int n = resident_count(D[i], boxes[sh][b]);
-          if (n <= 0 || n >= fewest) continue;
-          fewest = n;
-          front[i].push_back({boxes[sh][b].us, n, b});
-          bounds.push_back(boxes[sh][b].us);
-        }
+      if (same[i] < i) {
+        front[i] = front[same[i]];
+        continue;
       }
+      if ((long long)D[i].nx * D[i].ny * D[i].nz > most * box_voxels) continue;
+      // the fastest box of each count (some thousand boxes are looked at per volume: 120 pairs of different
+      // sizes take 6 ms of a set-up on three levels, 32 with divisions and branches for every box)
+      const auto &cx = counts[i][2], &cy = counts[i][1], &cz = counts[i][0];
+      float fastest[kResSlots + 1];  // [0]: counts that do not fit
+      int box_of[kResSlots + 1] = {};
+      std::fill(fastest, fastest + kResSlots + 1, 1e30f);
+      fastest[0] = -1.f;
+      for (int b = 0; b < (int)boxes.size();) {
+        const int end = boxes[b].next, nxy = cx[boxes[b].bx] * cy[boxes[b].by];
+        if (nxy > 0 && nxy <= most)
+          for (; b < end; ++b) {
+            int n = nxy * cz[boxes[b].bz];
+            n = n <= most ? n : 0;
+            const bool better = boxes[b].us < fastest[n];  // (selects: as branches they are mispredicted)
+            fastest[n] = better ? boxes[b].us : fastest[n];
+            box_of[n] = better ? b : box_of[n];
+          }
+        b = end;
+      }
+      float us = 1e30f;
+      for (int n = 1; n <= most; ++n)
+        if (fastest[n] < us) {
+          us = fastest[n];
+          front[i].push_back({us + launch, n, box_of[n]});
+          bounds.push_back(us + launch);
+        }
+      std::reverse(front[i].begin(), front[i].end());
     }
     std::sort(bounds.begin(), bounds.end());
     bounds.erase(std::unique(bounds.begin(), bounds.end()), bounds.end());
+    std::vector<int> fits, pick(np, -1);
+    for (int i = 0; i < np; ++i)
+      if (!front[i].empty()) {
+        fits.push_back(i);
+        pick[i] = 0;
+      }
+    const double rest = streamed(pick);  // the pairs left out
+    std::vector<int> at(np, -1);         // each pair's choice within the bound
     for (const float bound : bounds) {
-      std::vector<int> pick(np, -1);
       double total = 0.0;
       float longest = 0.f;
       int used = 0;
       bool ok = true;
-      for (int i = 0; i < np && ok; ++i) {
-        if (front[i].empty()) continue;
-        const Choice* c = nullptr;
-        for (const Choice& q : front[i])
-          if (q.us <= bound) c = &q;
-        if (!c) { ok = false; break; }
-        pick[i] = c->box;
-        const int takes = cluster ? 1 : c->count;
+      for (const int i : fits) {
+        while (at[i] + 1 < (int)front[i].size() && front[i][at[i] + 1].us <= bound) ++at[i];
+        if (at[i] < 0) {
+          ok = false;
+          break;
+        }
+        const Choice& c = front[i][at[i]];
+        const int takes = cluster ? 1 : c.count;
         if (used + takes > room) {
           total += longest;
           used = 0;
           longest = 0.f;
         }
         used += takes;
-        longest = std::max(longest, c->us);
+        longest = std::max(longest, c.us);
       }
-      total += longest;
       if (!ok) continue;
-      total += streamed(pick);  // the pairs left out
+      total += longest;
+      total += rest;
       if (best_us < 0 || total < best_us) {
         best_us = total;
         best_shape = sh;
-        best_box = pick;
+        best_box.assign(np, -1);
+        for (const int i : fits) best_box[i] = front[i][at[i]].box;
       }
     }
   }
   if (best_us < 0 || best_us >= streamed(std::vector<int>(np, -1))) return;
+  const std::vector<ResBoxes>& best_boxes = resident_boxes(P.prm.storage, best_shape);
   svs_plan::ResStep st;
   int npairs = 0, blocks = 0;  // blocks: of a cluster, a power of two
   if (kResCaps[best_shape].cluster) {
     blocks = 1;
     for (int i = 0; i < np; ++i)
-      while (best_box[i] >= 0 && blocks < resident_count(D[i], boxes[best_shape][best_box[i]])) blocks *= 2;
+      while (best_box[i] >= 0 && blocks < resident_count(D[i], best_boxes[best_box[i]])) blocks *= 2;
   }
   auto flush = [&] {
     if (npairs) P.res_steps[level].push_back(st);
@@ -1210,7 +1272,7 @@ void plan_resident(svs_plan& P, int level) {
   };
   for (int i = 0; i < np; ++i) {
     if (best_box[i] < 0) continue;
-    const ResBoxes& b = boxes[best_shape][best_box[i]];
+    const ResBoxes& b = best_boxes[best_box[i]];
     const int n = blocks ? blocks : resident_count(D[i], b);
     if (st.grid + n > (unsigned)(blocks ? kResSlots : slots)) flush();
     ResPair& r = st.launch.pair[npairs];
@@ -1227,7 +1289,7 @@ void plan_resident(svs_plan& P, int level) {
     st.launch.cluster = blocks;
     st.grid += (unsigned)n;
     st.threads = std::max(st.threads, (unsigned)ceil_div(b.threads, 32) * 32);
-    st.words = std::max(st.words, b.words);
+    st.words = std::max(st.words, (int)b.words);
     ++npairs;
     P.resident[level][i] = 1;
   }
