@@ -80,6 +80,7 @@ struct ResidentArgs {
   int src, dst;      // ping-pong copies read at the start and written at the end
   int iters;
   unsigned wait_us;  // bound of a wait for a neighbour
+  int mute;          // block that keeps its faces to itself (test hook of the waits), else -1
   int words;         // exchange words per box and field
   uint4* xbuf;       // [boxes][u, q][words]
   int* abort;        // raised when a wait gave up
@@ -459,6 +460,11 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       bar_init(bars + 8);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+  }
+  if (bid == a.mute) {
+#pragma unroll
+    for (int i = 0; i < C::NE; ++i)
+      if (word[i] >= 0) word[i] = -2;
   }
   auto arrived = [&](bool q, int it) {
     const unsigned bar = bars + (q ? 8 : 0);

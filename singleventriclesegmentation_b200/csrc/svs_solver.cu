@@ -605,6 +605,7 @@ struct svs_plan {
   // bounded pipeline waits (svs_tvl1_plan_set_stall_test)
   unsigned wait_us = 2000000;
   int stall_level = -1, stall_cta = -1, stall_plane = -1;
+  int mute_level = -1, mute_box = -1;      // the same for on-chip launches (svs_tvl1_plan_set_mute_test)
   // persistent iteration loop (svs_tvl1_plan_set_persistent): one cooperative launch per warp
   bool persistent = false;
   std::vector<char> level_persist;         // per level: the persistent form is used
@@ -1068,7 +1069,7 @@ struct ResBoxes {
 // Boxes that fit a compiled shape: x in pairs, z in whole groups of NP pairs (z fastest), the widest
 // first: of boxes that are modelled alike the first is taken, and of the same box in several orientations
 // the wide one is the faster (40^3 10x8x6 2.90 us per iteration, 8x6x10 2.98; 20^3 in a cluster 10x10x5
-// 1.80, 10x5x10 1.91; 12 x 40^3 f32 40x8x6 18.8, 6x8x40 22.6; the exception seen: 32^3 8x8x4 2.10, 4x8x8 2.04).
+// 1.80, 10x5x10 1.91; 12 x 40^3 f32 40x8x6 18.8, 6x8x40 22.6; 32^3 8x8x4 and 4x8x8 are alike: 2.10 and 2.04 on one GPU, 2.18 and 2.21 on another).
 std::vector<ResBoxes> list_boxes(int storage, const ResCaps& c) {
   std::vector<ResBoxes> out;
   for (int bx = kResMaxBx; bx >= 4; bx -= 2)
@@ -1328,6 +1329,7 @@ int resident_iterations(svs_plan& P, int level, int iters, int cur, cudaStream_t
     a.dst = cur ^ (iters & 1);
     a.iters = iters;
     a.wait_us = P.wait_us;
+    a.mute = level == P.mute_level ? P.mute_box : -1;
     a.words = st.words;
     a.xbuf = P.d_xbuf;
     a.abort = reinterpret_cast<int*>(reinterpret_cast<char*>(P.d_xbuf) + P.xbuf_bytes - 256);
@@ -2302,6 +2304,16 @@ svs_status svs_tvl1_plan_set_stall_test(svs_plan* P, int level, int cta, int pla
   P->stall_level = (level >= 0 && cta >= 0 && plane >= 0) ? level : -1;
   P->stall_cta = P->stall_level >= 0 ? cta : -1;
   P->stall_plane = P->stall_level >= 0 ? plane : -1;
+  P->wait_us = wait_us ? wait_us : 2000000u;
+  ++P->tile_epoch;  // the captured graph carries the launch arguments
+  return SVS_OK;
+}
+
+svs_status svs_tvl1_plan_set_mute_test(svs_plan* P, int level, int box, uint32_t wait_us) {
+  SVS_REQUIRE(P, "svs_tvl1_plan_set_mute_test: null plan");
+  SVS_REQUIRE(level < P->levels, "svs_tvl1_plan_set_mute_test: bad level");
+  P->mute_level = (level >= 0 && box >= 0) ? level : -1;
+  P->mute_box = P->mute_level >= 0 ? box : -1;
   P->wait_us = wait_us ? wait_us : 2000000u;
   ++P->tile_epoch;  // the captured graph carries the launch arguments
   return SVS_OK;

@@ -96,6 +96,12 @@ class SolverPlan:
         check() then raises with SVS_ERR_TIMEOUT. No arguments switch the stall off."""
         check(_lib.lib().svs_tvl1_plan_set_stall_test(self._h, int(level), int(cta), int(plane), int(wait_us)))
 
+    def set_mute_test(self, level: int = -1, box: int = -1, wait_us: int = 0) -> None:
+        """Test hook of the on-chip launches' bounded waits: CTA `box` of each such launch at `level` keeps
+        its faces to itself, so that its neighbours' waits run out after wait_us (0 = 2 s). No
+        arguments switch it off."""
+        check(_lib.lib().svs_tvl1_plan_set_mute_test(self._h, int(level), int(box), int(wait_us)))
+
     def retarget(self, dims: Sequence[Tuple[int, int, int]], stream=None) -> None:
         """Take another batch (at most as many pairs as at creation, state within the arena)
         without allocating; synchronizes `stream`."""
