@@ -351,6 +351,11 @@ svs_status svs_tvl1_chunk_plan(int64_t columns, int nz, int64_t slots, int* main
  * solves since the last check are invalid), SVS_OK otherwise. The status is cleared once it has
  * been reported. */
 svs_status svs_tvl1_plan_check(svs_plan* plan);
+/* The same for the plan's finished solves, without synchronising (a flag in host memory that the end
+ * of a solve writes): for a caller that has waited for a solve's results anyway. For a failure that
+ * neither call has reported, the plan's next svs_tvl1_solve_batch returns SVS_ERR_TIMEOUT, once and
+ * without solving, or svs_tvl1_plan_destroy does, having destroyed the plan. */
+svs_status svs_tvl1_plan_poll(svs_plan* plan);
 /* Test hook for the bounded pipeline waits of the TMA iterate kernels (no counterpart in the
  * reference): at pyramid `level`, the CTA with launch index `cta` never issues the copies of its
  * staged plane number `plane` (counted from the first plane it stages), and every pipeline wait

@@ -106,6 +106,7 @@ _SIGS = {
     "svs_tvl1_plan_set_mute_test": (c_int, [c_void_p, c_int, c_int, ctypes.c_uint32]),
     "svs_tvl1_plan_set_resident": (c_int, [c_void_p, c_int]),
     "svs_tvl1_chunk_plan": (c_int, [c_int64, c_int, c_int64, c_void_p, c_void_p, c_void_p]),
+    "svs_tvl1_plan_poll": (c_int, [c_void_p]),
     "svs_tvl1_plan_check": (c_int, [c_void_p]),
     "svs_tvl1_plan_set_stall_test": (c_int, [c_void_p, c_int, c_int, c_int, ctypes.c_uint32]),
     "svs_tvl1_plan_set_persistent": (c_int, [c_void_p, c_int]),

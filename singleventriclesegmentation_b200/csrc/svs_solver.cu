@@ -494,7 +494,8 @@ __global__ void residual_finish_kernel(const Desc* __restrict__ descs, double* _
 
 template <typename SU, typename SP>
 __global__ void finalize_kernel(const Desc* __restrict__ descs, int src, float* const* __restrict__ u_out,
-                                float* const* __restrict__ p_out) {
+                                float* const* __restrict__ p_out, const int* __restrict__ status, int* host_status) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && *status) *reinterpret_cast<volatile int*>(host_status) = *status;
   const Desc d = descs[blockIdx.y];
   const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (v >= d.n) return;
@@ -555,6 +556,7 @@ struct svs_plan {
   void* arena = nullptr;
   size_t arena_bytes = 0;
   int* d_status = nullptr;                 // device error bits (SVS_DEV_*)
+  int* h_status = nullptr;                 // the same in mapped host memory, written at the end of a solve
   float** d_raw = nullptr;                 // [2*pairs] raw input frames (device)
   float** d_uout = nullptr;                // [pairs] AoS u results
   float** d_pout = nullptr;                // [pairs] AoS p results (or null entries)
@@ -1647,7 +1649,7 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
     }
   }
   float** uo = q.median_kernel > 1 ? P.d_umed : P.d_uout;
-  finalize_kernel<SU, SP><<<grid(0), 256, 0, s>>>(D, cur, uo, P.d_pout);
+  finalize_kernel<SU, SP><<<grid(0), 256, 0, s>>>(D, cur, uo, P.d_pout, P.d_status, P.h_status);
   ++launches;
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
   if (q.median_kernel > 1) {
@@ -1849,6 +1851,8 @@ svs_status svs_tvl1_plan_create(const svs_tvl1_params* prm, int num_pairs, const
   if (!st) st = check_cuda(cudaMalloc((void**)&P->d_maps, (size_t)P->levels * num_pairs * sizeof(TMaps)), "svs_tvl1_plan_create");
   if (!st) st = check_cuda(cudaMalloc((void**)&P->d_status, sizeof(int)), "svs_tvl1_plan_create");
   if (!st) st = check_cuda(cudaMemset(P->d_status, 0, sizeof(int)), "svs_tvl1_plan_create");
+  if (!st) st = check_cuda(cudaHostAlloc((void**)&P->h_status, sizeof(int), cudaHostAllocMapped), "svs_tvl1_plan_create");
+  if (!st) *P->h_status = 0;
   if (st) { svs_tvl1_plan_destroy(P); return st; }
   // step-size schedule within a warp (tvl13d.py:208-211 reset, :240-249 update, host float64),
   // each value rounded to float as torch and pybind do.
@@ -1925,8 +1929,13 @@ svs_status svs_tvl1_plan_destroy(svs_plan* P) {
   cudaFree(P->d_snaps);
   for (float* p : P->snaps) cudaFree(p);
   cudaFree(P->arena);
+  // (cudaFree waited for the plan's solves)
+  const bool failed = P->h_status && (*reinterpret_cast<volatile int*>(P->h_status) & SVS_DEV_TIMEOUT);
+  cudaFreeHost(P->h_status);
   delete P;
-  return SVS_OK;
+  return failed ? fail(SVS_ERR_TIMEOUT, "svs_tvl1_plan_destroy: a wait inside a kernel of a solve of this plan timed out; "
+                                        "its results are invalid")
+                : SVS_OK;
 }
 
 size_t svs_tvl1_plan_device_bytes(const svs_plan* P) { return P ? P->arena_bytes : 0; }
@@ -2012,6 +2021,16 @@ svs_status svs_tvl1_plan_get_residuals(svs_plan* P, float* out, size_t count) {
   return check_cuda(cudaMemcpy(out, P->d_reslog, nlog * sizeof(float), cudaMemcpyDeviceToHost), "residuals");
 }
 
+// A finished solve of the plan gave up a wait and nobody was told: reported once, here.
+static svs_status take_status(svs_plan* P, cudaStream_t s, const char* what) {
+  volatile int* h = P->h_status;
+  if (!(*h & SVS_DEV_TIMEOUT)) return SVS_OK;
+  *h = 0;
+  const svs_status st = check_cuda(cudaMemsetAsync(P->d_status, 0, sizeof(int), s), what);
+  return st ? st : fail(SVS_ERR_TIMEOUT, std::string(what) + ": a wait inside a kernel of an earlier solve of this plan timed out; "
+                                         "its results are invalid");
+}
+
 svs_status svs_tvl1_solve_batch(svs_plan* P, const svs_pair_desc* pairs, int num_pairs,
                                 svs_stream_t stream) {
   SVS_REQUIRE(P && pairs, "svs_tvl1_solve_batch: null pointer");
@@ -2027,7 +2046,7 @@ svs_status svs_tvl1_solve_batch(svs_plan* P, const svs_pair_desc* pairs, int num
   }
   warm = warm && P->levels == 1;
   cudaStream_t s = stream;
-  svs_status st = SVS_OK;
+  svs_status st = take_status(P, s, "svs_tvl1_solve_batch");
   for (int i = 0; i < num_pairs && !st; ++i) {
     const size_t b = (size_t)P->h_descs[i].n * sizeof(float);
     st = check_cuda(cudaMemcpyAsync(P->raw[2 * i], pairs[i].I0, b, cudaMemcpyDeviceToDevice, s), "solve: input copy");
@@ -2196,12 +2215,19 @@ svs_status svs_tvl1_plan_check(svs_plan* P) {
   int flags = 0;
   svs_status st = check_cuda(cudaMemcpy(&flags, P->d_status, sizeof(int), cudaMemcpyDeviceToHost), "svs_tvl1_plan_check");
   if (st) return st;
+  flags |= *reinterpret_cast<volatile int*>(P->h_status);
   if (flags) {
+    *P->h_status = 0;
     st = check_cuda(cudaMemset(P->d_status, 0, sizeof(int)), "svs_tvl1_plan_check");  // reported once
     if (st) return st;
   }
   if (flags & SVS_DEV_TIMEOUT) return fail(SVS_ERR_TIMEOUT, "a pipeline wait in the iterate kernel timed out; results are invalid");
   return SVS_OK;
+}
+
+svs_status svs_tvl1_plan_poll(svs_plan* P) {
+  SVS_REQUIRE(P, "svs_tvl1_plan_poll: null plan");
+  return take_status(P, nullptr, "svs_tvl1_plan_poll");
 }
 
 svs_status svs_tvl1_plan_create_reserve(const svs_tvl1_params* prm, int max_pairs, size_t arena_bytes,

@@ -119,6 +119,7 @@ def process_patients(patients: Sequence[Tuple[str, torch.Tensor, int, int]], sol
                 writer.submit(out_dir, name, mode, process_sequence(img, tdia, tsys, mode, solver, median_kernel))
     finally:
         paths = writer.close()
+    solver.check()
     return paths
 
 

@@ -316,6 +316,7 @@ class FlowServer:
                 # finished batches: count their pairs; a request whose pairs are all done is finalized
                 for sl in self._slots:
                     if sl.batch and sl.event.query():
+                        sl.plan.poll()  # flows of a solve that gave up a wait are not handed out
                         for req, _ in sl.batch:
                             req.done += 1
                             if req.done == len(req.pairs):

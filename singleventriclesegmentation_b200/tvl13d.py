@@ -90,6 +90,12 @@ class SolverPlan:
         with torch.cuda.device(self.device):
             check(_lib.lib().svs_tvl1_plan_check(self._h))
 
+    def poll(self) -> None:
+        """check() for the solves that have finished, without synchronizing; what is not reported by
+        either is raised by the next solve(), or by close()."""
+        with torch.cuda.device(self.device):
+            check(_lib.lib().svs_tvl1_plan_poll(self._h))
+
     def set_stall_test(self, level: int = -1, cta: int = -1, plane: int = -1, wait_us: int = 0) -> None:
         """Test hook of the bounded pipeline waits: at `level`, CTA `cta` never issues the copies
         of its staged plane number `plane`, and waits give up after wait_us (0 = 2 s); the next
@@ -173,8 +179,8 @@ class SolverPlan:
 
     def close(self):
         if self._h:
-            _lib.lib().svs_tvl1_plan_destroy(self._h)
-            self._h = None
+            handle, self._h = self._h, None
+            check(_lib.lib().svs_tvl1_plan_destroy(handle))
 
     def __del__(self):
         try:
@@ -268,6 +274,13 @@ class TVL13DOpticalFlow:
         else:
             self._plans.move_to_end(key)
         return plan
+
+    def check(self) -> None:
+        """Raise if a bounded wait inside a kernel gave up in a solve whose flows have been returned
+        (synchronizes the device). Without it the next solve of the same sizes raises, before it starts."""
+        torch.cuda.synchronize(self.device)
+        for plan in self._plans.values():
+            plan.poll()
 
     @staticmethod
     def _frame(t: torch.Tensor, name: str) -> torch.Tensor:

@@ -43,3 +43,57 @@ def test_mute_box_times_out_and_the_plan_recovers(cuda, storage, shape, which, b
     plan.solve(*I, again)
     plan.check()
     assert torch.equal(again[0], ref[0])
+
+
+def make_solver(**kw):
+    return TVL13DOpticalFlow(1, 2, 24, 1.0, 0.025, 2, (0.5, 0.5, 0.25, 1.0), True, (5.0, 0.5), True, 1.0,
+                             "CUBIC_HERMITESPLINE", "MIRROR", "numDofs", (1, 1, 1), torch.device("cuda"), **kw)
+
+
+def test_callers_that_never_check_are_told(cuda):
+    """compute() of a solver: the next one raises, once; solver.check() does; and the plan's end does."""
+    shape = (24, 24, 24)
+    f = synthetic.frame_pair(shape, seed=11)
+    I = [torch.from_numpy(f[k]).cuda() for k in (0, 1)]
+    solver = make_solver(max_cached_plans=1)
+    ref = solver.compute(*I)[0]
+    plan = solver.plan_for([shape])
+    solver.check()
+    for report in (lambda: solver.compute(*I), solver.check, plan.poll):
+        plan.set_mute_test(level=0, box=3, wait_us=4000)
+        solver.compute(*I)
+        torch.cuda.synchronize()
+        plan.set_mute_test()
+        with pytest.raises(_lib.SVSError) as e:
+            report()
+        assert e.value.status == _lib.SVS_ERR_TIMEOUT
+        assert torch.equal(solver.compute(*I)[0], ref)
+        solver.check()
+    plan.set_mute_test(level=0, box=3, wait_us=4000)
+    solver.compute(*I)
+    with pytest.raises(_lib.SVSError) as e:
+        solver.compute(I[0][:20].contiguous(), I[1][:20].contiguous())  # the one cached plan makes room
+    assert e.value.status == _lib.SVS_ERR_TIMEOUT
+
+
+def test_patient_files_are_not_passed_off_as_good(cuda, tmp_path):
+    from singleventriclesegmentation_b200 import processor
+    img = torch.from_numpy(synthetic.cine_sequence(T=3, shape=(20, 24, 24), seed=2)).cuda()
+    solver = make_solver()
+    processor.process_patients([("a", img, 0, 2)], solver, str(tmp_path))
+    solver.plan_for([(20, 24, 24)] * 2).set_mute_test(level=0, box=1, wait_us=4000)
+    with pytest.raises(_lib.SVSError):
+        processor.process_patients([("b", img, 0, 2)], solver, str(tmp_path), modes=("forward",))
+
+
+def test_server_hands_out_no_flows_of_a_failed_solve(cuda):
+    from singleventriclesegmentation_b200.serving import FlowServer
+    srv = FlowServer(budget_bytes=8 << 30, solver_args=dict(num_scales=1, max_warps=1, max_outer_iterations=24),
+                     batch_voxels=4 * 24 ** 3, max_batch_pairs=4, num_plans=1)
+    frames = torch.from_numpy(synthetic.cine_sequence(T=3, shape=(24, 24, 24), seed=1))
+    srv.submit(frames).result(timeout=60)
+    srv._slots[0].plan.set_mute_test(level=0, box=2, wait_us=4000)
+    with pytest.raises(_lib.SVSError) as e:
+        srv.submit(frames).result(timeout=60)
+    assert e.value.status == _lib.SVS_ERR_TIMEOUT
+    srv.close()
