@@ -5,7 +5,8 @@ the only one under which iterations stay on the chip (any explicit variant means
 iteration).
 
 The variants are listed in include/svsflow.h (svs_tvl1_plan_set_tile). A level's "size class" is
-the multiset of its volume sizes; the cache key is (GPU name, storage, level sizes).
+the multiset of its volume sizes; the cache key is (GPU name, variants, storage, boundary, spacing,
+iterations per warp, level sizes).
 """
 from __future__ import annotations
 
@@ -46,10 +47,14 @@ def _variants_signature() -> str:
                     for i in map(_lib.tile_info, range(1, n + 1)))
 
 
-def _key(device, storage: str, level_dims) -> str:
+def _key(device, storage: str, level_dims, params) -> str:
+    """The GPU, the variants, the sizes, and what else the automatic choice and its time depend on:
+    boundary and spacing (which levels may stay on chip) and the iterations of a warp."""
     name = torch.cuda.get_device_name(device).replace(" ", "_")
     sig = ";".join("x".join(map(str, d)) for d in level_dims)
-    return f"{name}|{_variants_signature()}|{storage}|{sig}"
+    length = "unit" if params.length_type == 0 else f"{params.length_z:g}x{params.length_y:g}x{params.length_x:g}"
+    return (f"{name}|{_variants_signature()}|{storage}|{params.boundary},{length},"
+            f"{params.max_outer_iterations}|{sig}")
 
 
 def _load() -> Dict[str, int]:
@@ -162,7 +167,7 @@ def tune(plan: SolverPlan, storage: str, levels: int, candidates: Optional[Seque
     chosen = []
     lds = _level_dims(plan.dims, levels)
     for level in range(levels):
-        key = _key(plan.device, storage, [lds[level]])
+        key = _key(plan.device, storage, [lds[level]], plan.params)
         best = db.get(key)
         ranked = None
         if best is None or per_class:
