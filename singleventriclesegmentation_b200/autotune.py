@@ -24,11 +24,13 @@ from .tvl13d import SolverPlan
 CACHE = os.environ.get("SVS_AUTOTUNE_CACHE", os.path.join(os.path.expanduser("~"), ".cache", "svsflow", "autotune.json"))
 
 
-# An explicit variant replaces the automatic choice when it takes less than this part of its time. These
-# short timings do not reach the power cap that a long solve of streaming launches runs at, while
-# iterations on the chip stay below it: 68 pairs of 80^3 with FP32 storage timed 0.95 ms per
-# iteration with variant 13 and 1.0 ms automatically, but solved in 5.39 s and 5.20 s (1.66 and 1.97 GHz).
-AUTO_MARGIN = 0.92
+# Timings of a few iterations do not reach the power cap that a long solve of streaming launches may run
+# at, while iterations on the chip stay below it: 68 pairs of 80^3 with FP32 storage timed 0.95 ms per
+# iteration with variant 13 and 1.0 ms on chip, but solved in 5.39 s and 5.20 s (1.66 and 1.97 GHz). An
+# explicit variant that is faster than the on-chip form by less than this is timed against it
+# again, for long enough that the clocks settle.
+CLOSE = 0.92
+SETTLE_MS = 600.0
 
 
 def _level_dims(dims: Sequence[Tuple[int, int, int]], levels: int) -> List[List[Tuple[int, int, int]]]:
@@ -83,6 +85,11 @@ def _iters(plan: SolverPlan, tile: int, iters: int) -> int:
     return iters if tile else max(iters, int(plan.params.max_outer_iterations))
 
 
+def _settled_iters(plan: SolverPlan, ms: float) -> int:
+    per_warp = max(1, int(plan.params.max_outer_iterations))
+    return per_warp * max(1, int(np.ceil(SETTLE_MS / max(ms, 1e-3) / per_warp)))
+
+
 def time_variant(plan: SolverPlan, level: int, tile: int, iters: int = 6) -> Optional[float]:
     """Mean milliseconds per launch of `tile` at `level`, or None if the variant does not fit."""
     plan.set_level_tile(level, tile)
@@ -132,28 +139,41 @@ def _pair_level_dims(dims, level: int):
 def tune_classes(plan: SolverPlan, level: int, candidates: Sequence[int], iters: int = 6) -> Dict[int, int]:
     """Per size class of a level (pairs of equal width at that level): try `candidates` for the
     class's pairs while the others keep their variant, timing the whole level (the groups run
-    concurrently), and keep a class's choice when it is at least 2% faster. Returns
+    concurrently), and keep a class's choice when it is at least 2% faster. The first such choice takes
+    the whole level off the chip, so a close one (CLOSE) has to hold over a long timing as well. Returns
     {width: tile id} for the classes that left the level's variant."""
     ld = _pair_level_dims(plan.dims, level)
     widths = sorted({d[2] for d in ld})
     if len(widths) < 2:
         return {}
     base = time_level(plan, level, iters)
+    on_chip = plan.level_resident(level) > 0
     chosen = {}
     for w in widths:
         members = [i for i, d in enumerate(ld) if d[2] == w]
-        best_t, best_tid = base, 0
-        for t in candidates:
+
+        def assign(t):
             for i in members:
                 plan.set_pair_tile(level, i, t)
+
+        best_t, best_tid = base, 0
+        for t in candidates:
+            assign(t)
             ms = time_level(plan, level, iters)
             if ms is not None and ms < best_t * 0.98:
                 best_t, best_tid = ms, t
-        for i in members:
-            plan.set_pair_tile(level, i, best_tid)
+        if best_tid and on_chip and best_t > CLOSE * base:
+            n = _settled_iters(plan, base)
+            assign(best_tid)
+            off = time_level(plan, level, n)
+            assign(0)
+            if time_level(plan, level, n) * 0.98 <= off:
+                best_t, best_tid = base, 0
+        assign(best_tid)
         base = best_t
         if best_tid:
             chosen[w] = best_tid
+            on_chip = False
     return chosen
 
 
@@ -171,10 +191,19 @@ def tune(plan: SolverPlan, storage: str, levels: int, candidates: Optional[Seque
         best = db.get(key)
         ranked = None
         if best is None or per_class:
-            timings = {t: time_variant(plan, level, t, _iters(plan, t, iters)) for t in candidates}
-            timings = {t: v for t, v in timings.items() if v is not None}
-            ranked = sorted(timings, key=lambda t: timings[t] * (1.0 if t else AUTO_MARGIN))
-            best = ranked[0] if best is None else best
+            timings, on_chip = {}, False
+            for t in candidates:
+                ms = time_variant(plan, level, t, _iters(plan, t, iters))
+                if ms is not None:
+                    timings[t] = ms
+                    on_chip = on_chip or (t == 0 and plan.level_resident(level) > 0)
+            ranked = sorted(timings, key=timings.get)
+            if best is None:
+                best = ranked[0]
+                if on_chip and best != 0 and timings[best] > CLOSE * timings[0]:
+                    n = _settled_iters(plan, timings[best])
+                    if time_variant(plan, level, 0, n) <= time_variant(plan, level, best, n):
+                        best = 0
             db[key] = best
         plan.set_level_tile(level, best)
         chosen.append(best)

@@ -46,3 +46,58 @@ def test_cache_key_holds_what_the_choice_depends_on():
     assert len(keys) == 5
     # lengths say nothing where the spacing is one
     assert autotune._key(None, "f32", dims, params()) == autotune._key(None, "f32", dims, params(length_x=7.0))
+
+
+class Times:
+    """Stand-ins for the two timing functions: a level's ms per iteration by its requests, shortly after the
+    start (few iterations) and for good."""
+
+    def __init__(self, monkeypatch, short, settled):
+        self.short, self.settled, self.long_calls = short, settled, 0
+        monkeypatch.setattr(autotune, "time_variant", self.variant)
+        monkeypatch.setattr(autotune, "time_level", self.at)
+
+    def variant(self, plan, level, tile, iters=6):
+        plan.set_level_tile(level, tile)
+        return self.at(plan, level, iters)
+
+    def at(self, plan, level, iters=6):
+        long = iters * self.short[(0, 0)] >= autotune.SETTLE_MS
+        self.long_calls += long
+        tile, pairs = plan.requests(level)
+        return (self.settled if long else self.short).get((tile, max(pairs)))
+
+
+def tune(plan, levels=1, **kw):
+    return autotune.tune(plan, "f32", levels, candidates=[0, 3, 7], use_cache=False, **kw)
+
+
+def test_close_timings_are_settled_by_a_long_one(monkeypatch):
+    short = {(0, 0): 1.0, (3, 0): 0.95, (7, 0): 0.97}
+    t = Times(monkeypatch, short, {(0, 0): 1.0, (3, 0): 1.1, (7, 0): 1.1})
+    assert tune(Plan([(80, 80, 80)] * 2)) == [0] and t.long_calls == 2
+    t = Times(monkeypatch, short, {(0, 0): 1.0, (3, 0): 0.96, (7, 0): 1.1})
+    assert tune(Plan([(80, 80, 80)] * 2)) == [3]
+
+
+def test_no_margin_where_nothing_stays_on_chip(monkeypatch):
+    t = Times(monkeypatch, {(0, 0): 1.0, (3, 0): 0.95, (7, 0): 0.97}, {})
+    assert tune(Plan([(80, 80, 80)] * 2, resident=False)) == [3] and t.long_calls == 0
+
+
+def test_clear_timings_need_no_long_one(monkeypatch):
+    t = Times(monkeypatch, {(0, 0): 1.0, (3, 0): 0.9, (7, 0): 1.2}, {})
+    assert tune(Plan([(80, 80, 80)] * 2)) == [3] and t.long_calls == 0
+    t = Times(monkeypatch, {(0, 0): 1.0, (3, 0): 1.05, (7, 0): 1.2}, {})
+    assert tune(Plan([(80, 80, 80)] * 2)) == [0] and t.long_calls == 0
+
+
+def test_a_class_takes_a_level_off_the_chip_only_for_good(monkeypatch):
+    dims = [(40, 40, 40), (40, 40, 48)]
+    short = {(0, 0): 1.0, (3, 0): 1.2, (7, 0): 1.3, (0, 3): 0.95, (0, 7): 0.97}
+    for settled, left in (({(0, 0): 1.0, (0, 3): 0.99}, False), ({(0, 0): 1.0, (0, 3): 0.9}, True)):
+        Times(monkeypatch, short, settled)
+        plan = Plan(dims)
+        assert tune(plan, per_class=True) == [0]
+        assert bool(plan.class_tiles[0]) == left
+        assert (plan.level_resident(0) == 0) == left
