@@ -282,10 +282,12 @@ def tune_plan(plan, storage: str, levels: int = 3, per_class: bool = False):
 
 def iterate_roofline(plan, storage: str, level_voxels: int, stream, dev):
     """The dominant kernel (fused iteration, level 0) timed alone on the live state with CUDA
-    events: (ms per launch, algorithmic bytes per launch)."""
+    events: (ms per iteration, algorithmic bytes per iteration, pairs of the level on chip). Pairs on
+    chip run a warp's iterations per launch, so a whole warp is timed where there are any."""
     import torch
-    n_it = 30
     plan.bench_iterations(0, 3)
+    resident = plan.level_resident(0)
+    n_it = max(30, int(plan.params.max_outer_iterations)) if resident else 30
     torch.cuda.synchronize(dev)
     e4, e5 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e4.record(stream)
@@ -296,7 +298,22 @@ def iterate_roofline(plan, storage: str, level_voxels: int, stream, dev):
     # bytes per voxel-iteration: read u 3, p 9, D 6, rc 1, gw 3; write u 3, p 9
     ub = 2 if storage in ("bf16", "f16") else 4
     fb = 4 if storage == "f32" else 2
-    return it_ms, level_voxels * (6 * ub + 28 * fb)
+    return it_ms, level_voxels * (6 * ub + 28 * fb), resident
+
+
+def roofline_line(it_ms: float, alg: int, resident: int, kernel: str, traffic=None) -> dict:
+    """The roofline entry of a level's iterations. With one launch per iteration the bound is HBM: the
+    state's bytes over the measured peak. Pairs whose iterations stay on chip do not move that state, so
+    with any of them no fraction of HBM is stated."""
+    peak, kind = measured_peaks()
+    line = {"bound": "hbm", "achieved": alg / (it_ms / 1000.0) / 1e9, "peak": peak, "unit": "GB/s",
+            "frac": alg / (it_ms / 1000.0) / 1e9 / peak, "peak_kind": kind, "traffic": traffic, "kernel": kernel,
+            "algorithmic_bytes_per_launch": alg, "launch_ms": it_ms, "pairs_on_chip": resident}
+    if resident:
+        line.update({"bound": "latency and shared memory of the SMs (iterations on chip)", "achieved": None, "frac": None,
+                     "traffic": None, "algorithmic_bytes_per_launch": None,
+                     "kernel": "resident kernel, level 0 (launch_ms is per iteration)"})
+    return line
 
 
 def plain_form_rate(dev, seq_dev):
@@ -353,7 +370,7 @@ def pair_latency(dev, seq, storage: str, reps: int = 20):
 def fp32_storage_rate(dev, d_seq, pairs, args):
     """The same sequence solve with every iteration field stored in FP32 (the plain FP32 form of
     the fused path): pairs/s over 3 timed solves after autotuning, and the level-0 iterate
-    kernel's roofline fraction (136 algorithmic bytes per voxel-iteration)."""
+    kernel's roofline fraction (136 algorithmic bytes per voxel-iteration; none where it runs on chip)."""
     import torch
     solver = _solver(dev, "f32")
     n = len(pairs)
@@ -364,12 +381,12 @@ def fp32_storage_rate(dev, d_seq, pairs, args):
     I0s, I1s = [d_seq[a] for a, b in pairs], [d_seq[b] for a, b in pairs]
     ms, clocks = _timed_solves(plan, I0s, I1s, flows, 3, 2, dev)
     st = torch.cuda.current_stream(dev)
-    it_ms, alg = iterate_roofline(plan, "f32", n * int(np.prod(SHAPE)), st, dev)
-    peak, kind = measured_peaks()
+    line = roofline_line(*iterate_roofline(plan, "f32", n * int(np.prod(SHAPE)), st, dev), "iterate kernel, level 0")
     out = {"value": n / (ms / 1000.0), "unit": "pairs/s", "ms_per_step": ms, "steps": 3,
            "what": "the 68 pair solves alone (no mask propagation), FP32 storage of every field",
-           "level_tiles": plan.level_tiles()[:3], "launch_ms": it_ms,
-           "roofline_frac": alg / (it_ms / 1000.0) / 1e9 / peak, "peak_kind": kind, "clocks": clocks}
+           "level_tiles": plan.level_tiles()[:3], "level_resident": [plan.level_resident(l) for l in range(3)],
+           "launch_ms": line["launch_ms"], "roofline_frac": line["frac"], "bound": line["bound"],
+           "peak_kind": line["peak_kind"], "clocks": clocks}
     plan.close()
     solver._plans.clear()
     return out
@@ -447,8 +464,8 @@ def run_uneven(args):
     tiles = None if args.no_autotune else tune_plan(plan, args.storage, per_class=True)
     ms, clocks = _timed_solves(plan, I0s, I1s, outs, args.steps, args.warmup, dev)
     vox = sum(int(np.prod(d)) for d in dims)
-    it_ms, alg = iterate_roofline(plan, args.storage, vox, torch.cuda.current_stream(dev), dev)
-    peak, kind = measured_peaks()
+    line = roofline_line(*iterate_roofline(plan, args.storage, vox, torch.cuda.current_stream(dev), dev),
+                         "iterate kernels, level 0")
     print(json.dumps({
         "metric": "uneven-size TV-L1 flow pairs/s", "value": len(dims) / (ms / 1000.0), "unit": "pairs/s",
         "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,
@@ -458,8 +475,7 @@ def run_uneven(args):
                    "total_voxels": vox, "storage": args.storage, "level_tiles": plan.level_tiles()[:3],
                    "class_tiles": {str(l): {str(w): t for w, t in c.items()}
                                    for l, c in getattr(plan, "class_tiles", {}).items()}},
-        "roofline": {"bound": "hbm", "achieved": alg / (it_ms / 1000.0) / 1e9, "peak": peak, "unit": "GB/s",
-                     "frac": alg / (it_ms / 1000.0) / 1e9 / peak, "peak_kind": kind, "launch_ms": it_ms},
+        "roofline": line,
         "clocks": clocks}), flush=True)
 
 
@@ -752,10 +768,10 @@ def main():
 
     # ----- the dominant kernel (fused iteration, level 0) timed alone on the live state
     vox0 = n_pairs * int(np.prod(SHAPE))
-    it_ms, alg_bytes = iterate_roofline(plan, args.storage, vox0, stream, dev)
-    peak, peak_kind = measured_peaks()
-    achieved = alg_bytes / (it_ms / 1000.0) / 1e9
     traffic_pv = profiled_traffic().get(args.storage)
+    roofline = roofline_line(*iterate_roofline(plan, args.storage, vox0, stream, dev),
+                             "iterate kernel (fused primal-dual iteration, variant %d), level 0" % plan.level_tiles()[0],
+                             None if traffic_pv is None else traffic_pv * vox0)
 
     # the workload's own end metrics (warping.py:245-270): each propagated end mask against the
     # mask given at that end (two different synthetic annotations, so these are not parity values)
@@ -804,12 +820,7 @@ def main():
             "data": "synthetic", "config": config_dict(args, args.storage),
             "e2e": {"value": e2e_value, "unit": "pairs/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "peak_kind": peak_kind,
-                         "traffic": None if traffic_pv is None else traffic_pv * vox0,
-                         "kernel": "iterate kernel (fused primal-dual iteration, variant %d), level 0"
-                                   % plan.level_tiles()[0],
-                         "algorithmic_bytes_per_launch": alg_bytes, "launch_ms": it_ms},
+            "roofline": roofline,
             "cpu_baseline": cpu, "plain_gpu_form": plain, "clocks": clock_info, "latency": latency,
             "fp32_storage": fp32, "persistent_form": persistent, "compute_metrics": mask_metrics,
             "graph_kernels_per_solve": plan.graph_kernels,
