@@ -495,7 +495,9 @@ __global__ void residual_finish_kernel(const Desc* __restrict__ descs, double* _
 template <typename SU, typename SP>
 __global__ void finalize_kernel(const Desc* __restrict__ descs, int src, float* const* __restrict__ u_out,
                                 float* const* __restrict__ p_out, const int* __restrict__ status, int* host_status) {
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && *status) *reinterpret_cast<volatile int*>(host_status) = *status;
+  // (null in the allocation-free solve, whose kernels wait for nothing)
+  if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && *status)
+    *reinterpret_cast<volatile int*>(host_status) = *status;
   const Desc d = descs[blockIdx.y];
   const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (v >= d.n) return;
@@ -1047,12 +1049,12 @@ double stream_us(double work, bool groups) {
   return work <= 0.0 ? 0.0 : (10.0 + work * (1.0 + 0.25 / (1.0 + work / 100.0))) * (groups ? 1.15 : 1.0);
 }
 // A resident launch with boxes of `threads` threads of `np` voxel pairs and `words` face words:
-// the two exchanges (2.5 us with next to no work), the warps' pairs, the words' traffic, and the
-// launch itself over its iterations. 6x6x6 boxes 2.7 us, 8x8x10 3.4, 10x10x10 4.0 (np 1), 20x8x8
-// 4.6, 40x8x6 5.8, 20x10x10 6.2 (np 2; f32 5.3, 6.4 and 6.8), 20x12x15 9.7, 16x12x20 10.5 (np 5;
-// f32 13.8). In a cluster the exchanges take about 1.1 us: 9x11x12 in 8 boxes
-// 1.5 us, 20^3 in 16 boxes of 10x10x5 2.0, 18x21x24 in 16 2.45; the model is on the high side there, so that a tie
-// (24^3) goes to one box per SM.
+// the two exchanges, the warps' pairs and the words' traffic; launch_us is the launch itself over its
+// iterations. Modelled and measured (f16-flow32): 22x11x8 boxes (np 2) 5.8 and 5.8, 16x12x20 (np 5)
+// 10.55 and 10.5; f32 6.6 and 7.1, 13.85 and 13.8. The constants of the one-pair shapes date from before their
+// shrinkage step moved into the wait and their face words became two per thread: 6x4x4 boxes 2.7 and
+// 2.3, 10x8x6 3.4 and 2.9, 12x8x8 3.8 and 3.2, in a cluster 10x10x5 2.1 and 1.8. So the model is 15% on the
+// high side there, and batches of small pairs where both forms are that close stay per iteration.
 constexpr int kResMaxBx = 64, kResMaxByz = 48;  // of a box
 double launch_us(int iters) { return 6.0 / iters; }
 float resident_us(int storage, int np, int threads, int words, bool cluster) {
@@ -1313,8 +1315,9 @@ bool all_resident(const svs_plan& P, int level) {
 bool takes_turn(const svs_plan& P, int level) {
   if (P.prm.max_outer_iterations < 1 || P.prm.max_warps < 1) return false;
   if (level < (int)P.level_persist.size() && P.level_persist[level]) return true;
-  for (const svs_plan::ResStep& st : P.res_steps[level])
-    if (!kResCaps[st.shape].cluster) return true;
+  if (level < (int)P.res_steps.size())  // (empty in the allocation-free solve)
+    for (const svs_plan::ResStep& st : P.res_steps[level])
+      if (!kResCaps[st.shape].cluster) return true;
   return false;
 }
 
