@@ -1,5 +1,5 @@
-"""The general kernels of the resampling operators, which serve what the grid kernels do not: samples
-beyond the 32-bit coordinate range."""
+"""The general kernels of the resampling operators, which serve what the grid kernels do not: launches
+beyond a grid's limits (65,535 planes or volumes), and samples beyond the 32-bit coordinate range."""
 import numpy as np
 import pytest
 import torch
@@ -61,3 +61,51 @@ def test_far_samples_leave_the_other_gradients(cuda, interp, boundary):
     got, want = (op.backward(u, f.expand(nz, ny, nx, 3).contiguous(), torch.ones_like(u))[1] for f in (phi, near))
     ordinary = (which >= FAR.index(-2.5)).expand(nz, ny, nx)
     assert torch.equal(got[ordinary], want[ordinary])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("interp", ["NEAREST", "LINEAR", "CUBIC_HERMITESPLINE"])
+def test_tall_volumes(cuda, dtype, interp):
+    """Planes 10 to 19 of a tall volume (general kernel) and of its first 30 planes (grid kernel)."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    ny, nx, C = 5, 13, 3
+    u = torch.rand((TALL, ny, nx, C), generator=g, device="cuda", dtype=dtype)
+    phi = 4 * torch.rand((TALL, ny, nx, 3), generator=g, device="cuda", dtype=dtype) - 2
+    tol = 64 * torch.finfo(dtype).eps
+    kind = (getattr(of, "INTERPOLATE_" + interp), of.BOUNDARY_MIRROR)
+    for name, a in (("forward", u[..., 0].contiguous()), ("forwardVectorField", u)):
+        tall, few = (getattr(of.Warping3D(mesh(n, ny, nx), *kind), name)(a[:n].contiguous(), phi[:n].contiguous())[10:20]
+                     for n in (TALL, 30))
+        torch.testing.assert_close(tall, few, rtol=tol, atol=tol)
+    b = u[..., :2].permute(3, 0, 1, 2)[None]
+    tall, few = (of.WarpingCNN3D(mesh(n, ny, nx), *kind).forward(b[:, :, :n].contiguous(), phi[None, :n].contiguous())[:, :, 10:20]
+                 for n in (TALL, 30))
+    torch.testing.assert_close(tall, few, rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("interp", ["LINEAR", "CUBIC_HERMITESPLINE"])
+def test_many_volumes(cuda, interp):
+    g = torch.Generator(device="cuda").manual_seed(4)
+    n = 65540
+    u = torch.rand((n, 1, 3, 2, 4), generator=g, device="cuda")
+    phi = 3 * torch.rand((n, 3, 2, 4, 3), generator=g, device="cuda") - 1.5
+    op = of.WarpingCNN3D(mesh(3, 2, 4), getattr(of, "INTERPOLATE_" + interp), of.BOUNDARY_REFLECT)
+    tol = 64 * torch.finfo(torch.float32).eps
+    torch.testing.assert_close(op.forward(u, phi)[-40:], op.forward(u[-40:].contiguous(), phi[-40:].contiguous()), rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("interp", ["NEAREST", "LINEAR", "CUBIC_HERMITESPLINE"])
+def test_tall_targets(cuda, oracle, interp):
+    """A prolongation onto more planes than a grid has, with components padded and cropped."""
+    src, dst, C = (4, 3, 5), (TALL, 2, 3), 3
+    u = np.random.default_rng(5).standard_normal(src + (C,)).astype(np.float32)
+    op = of.Prolongation3D(mesh(*src), mesh(*dst), getattr(of, "INTERPOLATE_" + interp), of.BOUNDARY_MIRROR)
+    t = torch.from_numpy(u).cuda()
+    got = op.forwardVectorField(t)
+    want = oracle.prolongate(u, tuple(float(s - 1) for s in src), dst, tuple(float(s - 1) for s in dst), interp, "MIRROR")
+    if interp == "NEAREST":  # a target half way between two nodes may go to either
+        assert (np.abs(got.cpu().numpy() - want) > 2e-5).mean() < 1e-4
+    else:
+        np.testing.assert_allclose(got.cpu().numpy(), want, rtol=2e-5, atol=2e-5)
+    for n in (1, C, C + 2):
+        assert torch.equal(op.forwardVectorFieldPadded(t, n), torch.nn.functional.pad(got, (0, n - C)))
