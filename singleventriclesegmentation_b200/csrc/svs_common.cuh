@@ -125,9 +125,11 @@ __device__ __forceinline__ T sample_cubic(const FieldRefT<T>& f, T cz, T cy, T c
   return hermite4(bz[0], bz[1], bz[2], bz[3], wz);
 }
 
-// hermite4 inside its window (w + 1 below 2) with t = (w + 1) - 1 given. The roundings are hermite4's
-// as compiled: halves and doubles are exact, so (b2 - b0) / 2, 2 pf - 2 pc and their sums are kept as
-// differences and scaled where they are used; -3 pf + 3 pc is one product and one fused multiply-add.
+// hermite4 inside its window (w + 1 below 2) with t = (w + 1) - 1 given. The roundings are those of
+// hermite4 with its products fused into its sums: halves and doubles are exact, so (b2 - b0) / 2,
+// 2 pf - 2 pc and their sums are kept as differences and scaled where they are used; -3 pf + 3 pc is one
+// product and one fused multiply-add. (Exact down to the smallest normal floats: below them a half
+// taken early or late may differ in the last bit, as in the vanishing tails of long mask chains.)
 template <typename T> __device__ __forceinline__ T hermite_one(T b0, T b1, T b2, T b3, T t) {
   const T e0 = b2 - b0, e1 = b3 - b1;
   const T a2 = fma(T(4), b1 - b2, e0) + e1;

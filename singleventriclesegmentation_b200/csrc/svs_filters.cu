@@ -79,7 +79,8 @@ template <typename T> __device__ __forceinline__ void order(T& a, T& b) {
   b = tmax(a, b);
   a = lo;
 }
-// 25-comparator sorting network of 9 values.
+// Sorting network of 9 values: 25 comparators (the least possible) in 7 layers, from B. Dobbelaere's
+// published list of sorting networks.
 template <typename T> __device__ __forceinline__ void sort9(T (&w)[9]) {
   order(w[0], w[3]); order(w[1], w[7]); order(w[2], w[5]); order(w[4], w[8]);
   order(w[0], w[7]); order(w[2], w[4]); order(w[3], w[8]); order(w[5], w[6]);
