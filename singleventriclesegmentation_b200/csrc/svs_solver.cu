@@ -496,7 +496,7 @@ template <typename SU, typename SP>
 __global__ void finalize_kernel(const Desc* __restrict__ descs, int src, float* const* __restrict__ u_out,
                                 float* const* __restrict__ p_out, const int* __restrict__ status, int* host_status) {
   // (null in the allocation-free solve, whose kernels wait for nothing)
-  if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && *status)
+  if (host_status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && *status)
     *reinterpret_cast<volatile int*>(host_status) = *status;
   const Desc d = descs[blockIdx.y];
   const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -558,7 +558,8 @@ struct svs_plan {
   void* arena = nullptr;
   size_t arena_bytes = 0;
   int* d_status = nullptr;                 // device error bits (SVS_DEV_*)
-  int* h_status = nullptr;                 // the same in mapped host memory, written at the end of a solve
+  int* h_status = nullptr;                 // the same in host memory (StatusPage), written at the end of a solve
+  int* h_status_dev = nullptr;             // its device address (null: none)
   float** d_raw = nullptr;                 // [2*pairs] raw input frames (device)
   float** d_uout = nullptr;                // [pairs] AoS u results
   float** d_pout = nullptr;                // [pairs] AoS p results (or null entries)
@@ -1023,6 +1024,57 @@ class ResidentTurn {
   cudaStream_t s_;
   Turns* t_ = nullptr;
 };
+
+// One page of host memory that kernels can write, a word per plan: the status of a plan's finished solves
+// for callers that do not synchronise for it. Pinning memory takes 4 to 12 ms and giving it back as much, so
+// the page is pinned once, by the first plan, and stays so (4 KB); its words go from plan to plan. It is the
+// library's own memory, so that a device reset ends the mapping but not the page. Without a
+// word (more than 1024 plans at once, or no mapping) only svs_tvl1_plan_check reports.
+class StatusPage {
+ public:
+  static int* take(int** dev) {
+    *dev = nullptr;
+    std::lock_guard<std::mutex> lock(mutex());
+    void* d = nullptr;
+    if (cudaHostGetDevicePointer(&d, page(), 0) != cudaSuccess) {
+      cudaGetLastError();
+      if (cudaHostRegister(page(), kWords * sizeof(int), cudaHostRegisterPortable | cudaHostRegisterMapped) != cudaSuccess ||
+          cudaHostGetDevicePointer(&d, page(), 0) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+    }
+    for (int i = 0; i < kWords; ++i)
+      if (!used()[i]) {
+        used()[i] = true;
+        page()[i] = 0;
+        *dev = static_cast<int*>(d) + i;
+        return page() + i;
+      }
+    return nullptr;
+  }
+  static void give(int* word) {
+    if (!word) return;
+    std::lock_guard<std::mutex> lock(mutex());
+    used()[word - page()] = false;
+  }
+
+ private:
+  static constexpr int kWords = 1024;
+  static int* page() {
+    alignas(4096) static int p[kWords];
+    return p;
+  }
+  static bool* used() {
+    static bool u[kWords];
+    return u;
+  }
+  static std::mutex& mutex() {
+    static std::mutex m;
+    return m;
+  }
+};
+int host_flags(const svs_plan* P) { return P->h_status ? *reinterpret_cast<volatile int*>(P->h_status) : 0; }
 
 // Modelled microseconds per iteration, fitted to measurements on one B200.
 // The per-iteration kernels: what each pair's column tiles cost on a full GPU (the least of the
@@ -1652,7 +1704,7 @@ long long enqueue_solve(svs_plan& P, cudaStream_t s) {
     }
   }
   float** uo = q.median_kernel > 1 ? P.d_umed : P.d_uout;
-  finalize_kernel<SU, SP><<<grid(0), 256, 0, s>>>(D, cur, uo, P.d_pout, P.d_status, P.h_status);
+  finalize_kernel<SU, SP><<<grid(0), 256, 0, s>>>(D, cur, uo, P.d_pout, P.d_status, P.h_status_dev);
   ++launches;
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
   if (q.median_kernel > 1) {
@@ -1854,8 +1906,7 @@ svs_status svs_tvl1_plan_create(const svs_tvl1_params* prm, int num_pairs, const
   if (!st) st = check_cuda(cudaMalloc((void**)&P->d_maps, (size_t)P->levels * num_pairs * sizeof(TMaps)), "svs_tvl1_plan_create");
   if (!st) st = check_cuda(cudaMalloc((void**)&P->d_status, sizeof(int)), "svs_tvl1_plan_create");
   if (!st) st = check_cuda(cudaMemset(P->d_status, 0, sizeof(int)), "svs_tvl1_plan_create");
-  if (!st) st = check_cuda(cudaHostAlloc((void**)&P->h_status, sizeof(int), cudaHostAllocMapped), "svs_tvl1_plan_create");
-  if (!st) *P->h_status = 0;
+  if (!st) P->h_status = StatusPage::take(&P->h_status_dev);
   if (st) { svs_tvl1_plan_destroy(P); return st; }
   // step-size schedule within a warp (tvl13d.py:208-211 reset, :240-249 update, host float64),
   // each value rounded to float as torch and pybind do.
@@ -1933,8 +1984,8 @@ svs_status svs_tvl1_plan_destroy(svs_plan* P) {
   for (float* p : P->snaps) cudaFree(p);
   cudaFree(P->arena);
   // (cudaFree waited for the plan's solves)
-  const bool failed = P->h_status && (*reinterpret_cast<volatile int*>(P->h_status) & SVS_DEV_TIMEOUT);
-  cudaFreeHost(P->h_status);
+  const bool failed = host_flags(P) & SVS_DEV_TIMEOUT;
+  StatusPage::give(P->h_status);
   delete P;
   return failed ? fail(SVS_ERR_TIMEOUT, "svs_tvl1_plan_destroy: a wait inside a kernel of a solve of this plan timed out; "
                                         "its results are invalid")
@@ -2026,9 +2077,8 @@ svs_status svs_tvl1_plan_get_residuals(svs_plan* P, float* out, size_t count) {
 
 // A finished solve of the plan gave up a wait and nobody was told: reported once, here.
 static svs_status take_status(svs_plan* P, cudaStream_t s, const char* what) {
-  volatile int* h = P->h_status;
-  if (!(*h & SVS_DEV_TIMEOUT)) return SVS_OK;
-  *h = 0;
+  if (!(host_flags(P) & SVS_DEV_TIMEOUT)) return SVS_OK;
+  *P->h_status = 0;
   const svs_status st = check_cuda(cudaMemsetAsync(P->d_status, 0, sizeof(int), s), what);
   return st ? st : fail(SVS_ERR_TIMEOUT, std::string(what) + ": a wait inside a kernel of an earlier solve of this plan timed out; "
                                          "its results are invalid");
@@ -2218,9 +2268,9 @@ svs_status svs_tvl1_plan_check(svs_plan* P) {
   int flags = 0;
   svs_status st = check_cuda(cudaMemcpy(&flags, P->d_status, sizeof(int), cudaMemcpyDeviceToHost), "svs_tvl1_plan_check");
   if (st) return st;
-  flags |= *reinterpret_cast<volatile int*>(P->h_status);
+  flags |= host_flags(P);
   if (flags) {
-    *P->h_status = 0;
+    if (P->h_status) *P->h_status = 0;
     st = check_cuda(cudaMemset(P->d_status, 0, sizeof(int)), "svs_tvl1_plan_check");  // reported once
     if (st) return st;
   }

@@ -20,7 +20,7 @@ def test_choice_is_a_small_part_of_a_set_up(cuda):
     plan = SolverPlan.reserve(solver.params(), 120, 24 << 30, torch.device("cuda"))
     rng = random.Random(0)
     best = {}
-    for repeat in range(4):
+    for repeat in range(8):
         dims = [tuple(rng.randrange(24, 97) for _ in range(3)) for _ in range(120)]
         I = [torch.zeros(d, device="cuda") for d in dims]
         outs = [torch.empty(d + (3,), device="cuda") for d in dims]
