@@ -91,10 +91,15 @@ using FieldRef = FieldRefT<float>;
 
 // Grid coordinate -> (floor index, fraction), the reference's floorf(c/h) and c/h - floor.
 template <typename T>
-__device__ __forceinline__ void split_coord(T c, T h, int& i, T& w) {
+__device__ __forceinline__ void split_saturated(T c, T h, int& k, T& w) {
   const T g = h == T(1) ? c : c / h;
-  const int k = floor_index(g);
+  k = floor_index(g);
   w = g - (T)k;
+}
+template <typename T>
+__device__ __forceinline__ void split_coord(T c, T h, int& i, T& w) {
+  int k;
+  split_saturated(c, h, k, w);
   i = safe_index(k);
 }
 
@@ -181,14 +186,17 @@ template <typename T>
 __device__ __forceinline__ CubicTaps<T> cubic_taps(T cz, T cy, T cx, T hz, T hy, T hx) {
   CubicTaps<T> k;
   T wx, wy, wz;
-  split_coord(cx, hx, k.x, wx);
-  split_coord(cy, hy, k.y, wy);
-  split_coord(cz, hz, k.z, wz);
+  split_saturated(cx, hx, k.x, wx);
+  split_saturated(cy, hy, k.y, wy);
+  split_saturated(cz, hz, k.z, wz);
   const T lx = wx + T(1), ly = wy + T(1), lz = wz + T(1);
   k.tx = lx - T(1);
   k.ty = ly - T(1);
   k.tz = lz - T(1);
-  k.plain = lx >= T(1) && lx < T(2) && ly >= T(1) && ly < T(2) && lz >= T(1) && lz < T(2);
+  // (w is below 0 only where the index saturated; two comparisons leave those out with all whose taps'
+  // indices could overflow)
+  k.plain = lx < T(2) && ly < T(2) && lz < T(2) && min(min(k.x, k.y), k.z) > -0x7fffff00 &&
+            max(max(k.x, k.y), k.z) < 0x7fffff00;
   if (k.plain) --k.x, --k.y, --k.z;
   return k;
 }
