@@ -1122,25 +1122,34 @@ struct ResBoxes {
   int next;  // first box of another (x, y) extent
   float us;  // modelled time per iteration, less the launch's part
 };
-// Boxes that fit a compiled shape: x in pairs, z in whole groups of NP pairs (z fastest), the widest
-// first: of boxes that are modelled alike the first is taken, and of the same box in several orientations
-// the wide one is the faster (40^3 10x8x6 2.90 us per iteration, 8x6x10 2.98; 20^3 in a cluster 10x10x5
-// 1.80, 10x5x10 1.91; 12 x 40^3 f32 40x8x6 18.8, 6x8x40 22.6; 32^3 8x8x4 and 4x8x8 are alike: 2.10 and 2.04 on one GPU, 2.18 and 2.21 on another).
+// Boxes that fit a compiled shape: x in pairs, z in whole groups of NP pairs (z fastest). Of boxes that are
+// modelled alike, as the orientations of one box are, the first is taken. One pair per thread, one box per
+// SM: the tallest along y, then along z (32x38x16 f32 4x8x5 (z y x) 2.31 us per iteration, the others 2.32-2.40;
+// 31x24x46 2.23, 2.24-2.37; 40^3 2.75, 2.77-2.90; 48^3 3.15, 3.06-3.15; 32^3 2.21, 2.17-2.24). The others: the
+// widest along x, then along y (12 x 40^3 f32, two pairs per thread, 18.4 us, 18.8-22.9; 20^3 in a cluster
+// 1.61, up to 1.71; 4 x 24^3 in clusters 2.27, 2.26-2.43).
 std::vector<ResBoxes> list_boxes(int storage, const ResCaps& c) {
   std::vector<ResBoxes> out;
-  for (int bx = kResMaxBx; bx >= 4; bx -= 2)
+  auto along_z = [&](int bx, int by) {
+    for (int bz = std::max(2, c.np); bz <= kResMaxByz; bz += c.np) {
+      const int threads = bx / 2 * by * (bz / c.np);
+      const int words = 2 * (bz * by + bz * bx + by * bx);
+      if (threads > c.nt) break;
+      if (words > c.ne * (int)ceil_div(threads, 32) * 32) continue;
+      const int col = 2 * bz * by;
+      if ((bz + 2) * (by + 2) * bx + col > c.cu || std::max(bz * by * bx + col, std::max(bz * (by + 2) * bx, (bz + 2) * by * bx)) > c.cq)
+        continue;
+      out.push_back({(unsigned char)bx, (unsigned char)by, (unsigned char)bz, (short)threads, (short)words, 0,
+                     resident_us(storage, c.np, threads, words, c.cluster)});
+    }
+  };
+  if (c.np == 1 && !c.cluster) {
     for (int by = kResMaxByz; by >= 2; --by)
-      for (int bz = std::max(2, c.np); bz <= kResMaxByz; bz += c.np) {
-        const int threads = bx / 2 * by * (bz / c.np);
-        const int words = 2 * (bz * by + bz * bx + by * bx);
-        if (threads > c.nt) break;
-        if (words > c.ne * (int)ceil_div(threads, 32) * 32) continue;
-        const int col = 2 * bz * by;
-        if ((bz + 2) * (by + 2) * bx + col > c.cu || std::max(bz * by * bx + col, std::max(bz * (by + 2) * bx, (bz + 2) * by * bx)) > c.cq)
-          continue;
-        out.push_back({(unsigned char)bx, (unsigned char)by, (unsigned char)bz, (short)threads, (short)words, 0,
-                       resident_us(storage, c.np, threads, words, c.cluster)});
-      }
+      for (int bx = 4; bx <= kResMaxBx; bx += 2) along_z(bx, by);  // (narrow x: of one box's orientations the deep z)
+  } else {
+    for (int bx = kResMaxBx; bx >= 4; bx -= 2)
+      for (int by = kResMaxByz; by >= 2; --by) along_z(bx, by);
+  }
   for (int b = (int)out.size() - 1, next = b + 1; b >= 0; --b) {
     if (b + 1 < (int)out.size() && (out[b].bx != out[b + 1].bx || out[b].by != out[b + 1].by)) next = b + 1;
     out[b].next = next;
