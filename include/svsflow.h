@@ -364,8 +364,9 @@ svs_status svs_tvl1_plan_poll(svs_plan* plan);
  * svs_tvl1_plan_check reports SVS_ERR_TIMEOUT; the context stays usable. level, cta or plane < 0
  * switches the stall off (wait_us still applies). */
 svs_status svs_tvl1_plan_set_stall_test(svs_plan* plan, int level, int cta, int plane, uint32_t wait_us);
-/* The same for iterations on chip: CTA `box` of every on-chip launch at `level` never passes its faces on (it still waits for its neighbours' within a cluster), and waits
- * give up after wait_us. level or box < 0 switches it off. */
+/* The same for iterations on chip: CTA `box` of every on-chip launch at `level` never passes its faces
+ * on (within a cluster it still waits for its neighbours'), and waits give up after wait_us. level or
+ * box < 0 switches it off. FP32 and f16-flow32 storage only. */
 svs_status svs_tvl1_plan_set_mute_test(svs_plan* plan, int level, int box, uint32_t wait_us);
 /* Persistent iteration loop (no counterpart in the reference, whose tvl13d.py:213-253 launches
  * every operator of every iteration): with on != 0, each warp of a level whose pairs all use one

@@ -80,8 +80,8 @@ struct ResidentArgs {
   int src, dst;      // ping-pong copies read at the start and written at the end
   int iters;
   unsigned wait_us;  // bound of a wait for a neighbour
-  int mute;          // block that keeps its faces to itself (test hook of the waits), else -1
   int words;         // exchange words per box and field
+  int mute;          // MUTE: block that keeps its faces to itself (test hook of the waits), else -1
   uint4* xbuf;       // [boxes][u, q][words]
   int* abort;        // raised when a wait gave up
 };
@@ -96,10 +96,13 @@ struct ResidentArgs {
 // EARLY: the part of the primal that needs no q, the step of the shrinkage, is computed between publishing q's
 // faces and waiting for the neighbours' (35x41x47 f16-flow32 3.43 -> 3.27 us, 40^3 3.37 -> 3.2, 20^3 2.0 -> 1.83). The
 // 5-pair shape is short of registers for it (10.6 -> 11.0, f32 13.8 -> 15.7).
-template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_D_, bool KEEP_R_, bool CLUSTER_ = false>
+// MUTE: the form with the test hook of the waits (ResidentArgs::mute), apart because its one comparison
+// cost the cluster form 2% by other registers (f32 9x11x12 1.132 -> 1.158 us).
+template <int NP_, int NT_, int CU_, int CQ_, int NE_, bool KEEP_D_, bool KEEP_R_, bool CLUSTER_ = false, bool MUTE_ = false>
 struct ResShape {
   static constexpr int NP = NP_, NT = NT_, CU = CU_, CQ = CQ_, NE = NE_;
-  static constexpr bool CLUSTER = CLUSTER_, EARLY = NP <= 2;
+  static constexpr bool CLUSTER = CLUSTER_, EARLY = NP <= 2, MUTE = MUTE_;
+  using WithMute = ResShape<NP_, NT_, CU_, CQ_, NE_, KEEP_D_, KEEP_R_, CLUSTER_, true>;
   static constexpr bool KEEP_D = KEEP_D_, KEEP_R = KEEP_R_, ROLL = !KEEP_D;
   // the register file holds 16,384 registers per scheduler, a quarter of the warps each
   static constexpr int WARPS = (NT + 31) / 32, MAXREG = 16384 / ((WARPS + 3) / 4 * 32) / 8 * 8;
@@ -461,10 +464,12 @@ resident_kernel(const __grid_constant__ ResLaunch L, const Desc* __restrict__ de
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
   }
-  if (bid == a.mute) {
+  if constexpr (C::MUTE) {
+    if (bid == a.mute) {
 #pragma unroll
-    for (int i = 0; i < C::NE; ++i)
-      if (word[i] >= 0) word[i] = -2;
+      for (int i = 0; i < C::NE; ++i)
+        if (word[i] >= 0) word[i] = -2;
+    }
   }
   auto arrived = [&](bool q, int it) {
     const unsigned bar = bars + (q ? 8 : 0);
@@ -700,8 +705,49 @@ constexpr ResCaps kResCaps[kResShapes] = {res_caps<ResSmall>(), res_caps<ResMid>
 
 // op 0: set the kernel's attributes and return in *occ the CTAs one SM holds, or the clusters of
 // kResClusterBlocks CTAs that the GPU holds (false: not usable); op 1: one launch of `grid` CTAs of `threads`
-// threads on stream s, cooperative or in clusters of L->cluster.
+// threads on stream s, cooperative or in clusters of L->cluster. With a->mute set the launch takes the form
+// with the hook (FP32 and f16-flow32 storage; false for the others).
 bool resident_variant(int storage, int shape, int op, unsigned grid, unsigned threads, const ResLaunch* L,
                       const Desc* descs, const ResidentArgs* a, int* status, cudaStream_t s, int* occ);
+bool resident_mute(int storage, int shape, int op, unsigned grid, unsigned threads, const ResLaunch* L, const Desc* descs,
+                   const ResidentArgs* a, int* status, cudaStream_t s, int* occ);
+
+// Attributes or launch of one instantiation (op as above).
+template <typename SU, typename SP, typename C>
+bool resident_run(int op, unsigned grid, unsigned threads, const ResLaunch* L, const Desc* descs, const ResidentArgs* a,
+                  int* status, cudaStream_t s, int* occ) {
+  const auto k = resident_kernel<SU, SP, C>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if constexpr (C::CLUSTER) {
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = op ? L->cluster : kResClusterBlocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  } else {
+    // its CTAs wait for one another: a cooperative launch starts only a grid that fits the GPU at once
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+  }
+  if (op == 0) {
+    bool ok = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) == cudaSuccess;
+    if constexpr (C::CLUSTER) {
+      cfg.gridDim = dim3(kResClusterBlocks);
+      cfg.blockDim = dim3(C::NT);
+      ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+           cudaOccupancyMaxActiveClusters(occ, k, &cfg) == cudaSuccess;
+    } else {
+      ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, C::NT, C::SMEM) == cudaSuccess;
+    }
+    if (!ok) cudaGetLastError();
+    return ok && *occ > 0;
+  }
+  return cudaLaunchKernelEx(&cfg, k, *L, descs, *a, status) == cudaSuccess;
+}
 
 }  // namespace svs

@@ -2400,6 +2400,8 @@ svs_status svs_tvl1_plan_set_stall_test(svs_plan* P, int level, int cta, int pla
 svs_status svs_tvl1_plan_set_mute_test(svs_plan* P, int level, int box, uint32_t wait_us) {
   SVS_REQUIRE(P, "svs_tvl1_plan_set_mute_test: null plan");
   SVS_REQUIRE(level < P->levels, "svs_tvl1_plan_set_mute_test: bad level");
+  SVS_REQUIRE(level < 0 || box < 0 || P->prm.storage == SVS_STORAGE_F32 || P->prm.storage == SVS_STORAGE_F16_FLOW32,
+              "svs_tvl1_plan_set_mute_test: compiled for FP32 and f16-flow32 storage");
   P->mute_level = (level >= 0 && box >= 0) ? level : -1;
   P->mute_box = P->mute_level >= 0 ? box : -1;
   P->wait_us = wait_us ? wait_us : 2000000u;
