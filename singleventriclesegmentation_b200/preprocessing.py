@@ -7,6 +7,7 @@ rounded (prolongation.py:81-82), and the time axis zero-padded to pad_time frame
 """
 from __future__ import annotations
 
+import numbers
 from typing import Optional, Tuple
 
 import torch
@@ -44,6 +45,9 @@ def resample_patient(img_zyxt: torch.Tensor, seg_dia_zyx: Optional[torch.Tensor]
     seg_dia = op.forward(seg_dia_zyx.float().contiguous()).round() if seg_dia_zyx is not None else None
     seg_sys = op.forward(seg_sys_zyx.float().contiguous()).round() if seg_sys_zyx is not None else None
     img = img_zyxt.float().contiguous()
-    img = op.forwardVectorFieldPadded(img, pad_time) if pad_time > 0 else time_pading(pad_time, op.forwardVectorField(img))
+    if isinstance(pad_time, numbers.Integral) and pad_time > 0:
+        img = op.forwardVectorFieldPadded(img, pad_time)
+    else:  # (refuses what is no frame count)
+        img = time_pading(pad_time, op.forwardVectorField(img))
     factors = (NX / nx, NY / ny, NZ / nz, pad_time / nt)
     return img, seg_dia, seg_sys, factors

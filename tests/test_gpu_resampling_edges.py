@@ -54,3 +54,15 @@ def test_prolongation_edges(cuda, oracle, of, interp, src, dst, C):
     np.testing.assert_allclose(got.cpu().numpy(), want, rtol=2e-5, atol=2e-5)
     for n in (1, C, C + 6):
         assert torch.equal(op.forwardVectorFieldPadded(T(u), n), torch.nn.functional.pad(got, (0, n - C)))
+
+
+def test_frame_counts_that_are_none_are_refused(cuda):
+    """A fraction of a frame, which torch's pad refuses; any integer type is one."""
+    from singleventriclesegmentation_b200.preprocessing import resample_patient
+    img = torch.rand(5, 6, 7, 4, device="cuda")
+    want = resample_patient(img, shape=(6, 6, 6), pad_time=6)[0]
+    assert tuple(want.shape) == (6, 6, 6, 6)
+    assert torch.equal(resample_patient(img, shape=(6, 6, 6), pad_time=np.int64(6))[0], want)
+    for t in (6.0, 6.5, "6"):
+        with pytest.raises(TypeError):
+            resample_patient(img, shape=(6, 6, 6), pad_time=t)
