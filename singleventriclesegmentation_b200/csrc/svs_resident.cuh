@@ -32,13 +32,13 @@
 // another pair is waited for, so the launch is not cooperative. An exchange takes about 0.55 us instead of 1.25
 // (0.75 with a cluster barrier per exchange, whose release waits until the stores have arrived):
 // 20^3 2.8 -> 2.0 us per iteration (16 boxes of 10x10x5), 9x11x12 2.7 -> 1.5, 18x21x24 2.85 -> 2.45
-// (1.9, 1.35 and 2.2 with EARLY below; f32 1.8, 1.22 and 2.07). From about
+// (1.8, 1.25 and 2.2 with EARLY and two word slots, below; f32 1.7, 1.13 and 2.06). From about
 // 200 voxel pairs per box on, the boxes' arithmetic is worth more than that (24^3: 2.6 us on 144 SMs),
 // and the choice in plan_resident sees it.
 //
 // Measured on one B200 (us per iteration; before: one launch per iteration, march along z):
-//   f16-flow32 80^3 10.6 (20.4), 48^3 3.1 (14.4), 40^3 3.0 (10.3), 20^3 1.9 (8.2);
-//   f32 80^3 13.8 (20.5), 48^3 3.1 (12.3), 20^3 1.8 (10.3); 12 pairs of 40^3 f16-flow32 17.2 (26.7).
+//   f16-flow32 80^3 10.5 (20.4), 48^3 3.2 (14.4), 40^3 2.85 (10.3), 20^3 1.8 (8.2);
+//   f32 80^3 13.8 (20.5), 48^3 3.15 (12.3), 20^3 1.7 (10.3); 12 pairs of 40^3 f16-flow32 16.1 (26.7).
 // Small boxes are bound by the two exchanges (about 2.5 us: publish, poll, barriers). 80^3 is
 // bound by the latency of 12 warps of 168 registers (about 8,000 cycles of dual, 5,800 of primal)
 // and by the words' L2 traffic (3.6 MB per exchange each way). Its f32 form keeps p alone (90
